@@ -1,14 +1,13 @@
 // unet3d.cu — kernels of the learned warm start (include/unet3d.h): 3x3x3
-// convolutions as implicit GEMMs on the BF16 tensor cores (mma.sync m16n8k16,
-// FP32 accumulation), their data and weight gradients, 2x pooling / upsampling with
+// convolutions as implicit GEMMs on the BF16 tensor cores (FP32 accumulation), their data and weight gradients, 2x pooling / upsampling with
 // skip concatenation, the masked MSE loss and Adam.
 //
-// Forward (and data-gradient) convolution: one warp computes a tile of 16
-// consecutive voxels along x by all output channels.  The K loop runs over the 27
-// taps and 16-channel slices of the input; A fragments are read straight from the
-// channels-last activations (each thread loads the 32-bit channel pairs of two
-// voxels), B fragments from the [tap][Cout][Cin] weights, both through the read-only
-// cache.  Taps whose row lies outside the box are skipped warp-uniformly; voxels
+// Forward (and data-gradient) convolution: halo tiles on tcgen05 (conv_halo_kernel).  The
+// warp tiles (conv_fwd_kernel, mma.sync) take tensors that are not 16-byte aligned and are an
+// engine of their own: one warp computes 16 consecutive voxels along x by all output
+// channels, K runs over the 27 taps and 16-channel slices, A fragments come straight from the
+// channels-last activations, B fragments from the [tap][Cout][Cin] weights, both through the
+// read-only cache.  Taps whose row lies outside the box are skipped warp-uniformly; voxels
 // outside the row read zero.
 //
 // Weight gradient: dW[tap] = dY^T X_shift is a GEMM whose reduction runs over the
@@ -23,6 +22,7 @@
 #include <cudaTypedefs.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <string>
@@ -148,16 +148,10 @@ __global__ void __launch_bounds__(128) conv_fwd_kernel(const bf16* __restrict__ 
   }
 }
 
-// ---- forward convolution on the 5th-generation tensor cores (tcgen05) ----------------
-// A CTA owns 128 consecutive voxels (M = 128) and all output channels (N = Cout); the
-// K loop runs over 27 taps x 16-channel slices, one tcgen05.mma (K = 16) each.  Every
-// thread gathers its voxel's 16 channels of the tap's neighbour into the A tile and the
-// CTA copies the tap's 16 x Cout weights into the B tile, both in the K-major
-// "interleaved" core-matrix layout (8 rows x 16 bytes per core matrix); two stages, so
-// the next gather overlaps the running MMA.  One thread issues the MMA and commits it
-// to the stage's mbarrier; the FP32 accumulator lives in tensor memory (TMEM) and is
-// read back with tcgen05.ld for the bias / ReLU / BF16 epilogue.  Every wait is
-// bounded: a wait that gives up sets the error word and the CTA still frees its TMEM.
+// ---- tcgen05: descriptors and bounded waits --------------------------------------------
+// MMAs are issued by one thread and committed to an mbarrier; accumulators live in tensor
+// memory (TMEM).  Every wait is bounded: a wait that gives up sets the error word and the
+// block still frees its TMEM.
 constexpr int TC_M = 128;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -173,6 +167,15 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint
 // Instruction descriptor of kind::f16: BF16 A and B (K-major), FP32 accumulator, M x N.
 __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
+// One lane of a converged warp.  MMA loops run under it rather than under `lane == 0`: the
+// compiler then knows that one thread is active and keeps the descriptors in uniform
+// registers (measured on B200 with N = 48: 45 cycles per MMA against 68 to 117).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+  return e != 0u;
 }
 
 __device__ __forceinline__ void tc_mbar_init(uint64_t* bar) {
@@ -210,21 +213,133 @@ __global__ void __launch_bounds__(32) tc_wait_probe_kernel(const int polls, int*
   if (!__all_sync(0xffffffffu, ok) && threadIdx.x == 0) atomicExch(err, 1);
 }
 
+// ---- forward convolution on halo tiles (tcgen05) --------------------------------------
+// The input of a tile is staged once in shared memory with its one-voxel halo, and the 27
+// taps are 27 start addresses into it.  Axes: x, P (16 voxels per tile) and R (a run of
+// `br` planes); P and R are y and z or, where that leaves fewer voxels of padding, z and y.
+//   A operand: the slab keeps a 16-channel slice as two planes of 8 channels (16 bytes) per
+//     voxel, so 8 x-neighbours are one 128-byte core matrix of the K-major interleaved
+//     layout, the 16 rows along P are 8-row groups one slab row apart (stride byte offset),
+//     and the channel halves are one plane apart (leading byte offset).  A tap only moves
+//     the start address.  A matrix is 8 (x) by 16 (P) voxels, M = 128, no padding rows.
+//   D accumulator: the planes along R of one x group lie side by side in tensor memory.  An
+//     input plane contributes to three output planes, so one MMA with N = 3 Cout (the
+//     three R taps of one (P, x) tap side by side in the B operand) adds to all three:
+//     9 MMAs per input plane and slice instead of 27 per output plane.
+// What bounds it: an MMA with M = 128 reads 4 KB of A and 32 N bytes of B from shared memory,
+// 33 + N / 4 cycles, against N / 2 of arithmetic; with Cout = 16 an MMA of N = 16 costs 40
+// cycles and one of N = 48, three times the work, 45.
+// Loads (cp.async, zero fill outside the box), MMAs and the epilogue of successive tiles run
+// side by side: two slabs, two accumulators, one barrier per slice.  One block per SM.
+// Measured (B200, 4 x 64 x 64 x 128 voxels): 16 -> 16 channels 592 us with the warp tiles, 52
+// here; 48 -> 16 about 1700 -> 136; 96 -> 32 at 4 x 32 x 32 x 64 225 us (threads gathering
+// every tap of 128 voxels into shared memory) -> 60; 64 -> 64 at 4 x 16 x 16 x 32 94 -> 20.
+constexpr int HT_LOADERS = 256;                // load and epilogue threads (8 warps)
+constexpr int HT_THREADS = HT_LOADERS + 32;    // plus the warp that issues the MMAs
+constexpr int HT_P = 16;                       // voxels of a tile along P
+constexpr int HT_MAX_SMEM = 227 * 1024 - 1024; // dynamic part; the rest is static
+
+struct HaloArgs {
+  int n, np, nr, w;              // box: batch, P, R, x
+  long long sp, sr, sn;          // strides in voxels
+  int tap_p, tap_r;              // strides of P and R in the tap index (3 or 9)
+  int cin, kcs;                  // input channels and 16-channel slices
+  int br;                        // output planes of a tile along R
+  int tx, tp, tr;                // tiles per axis
+  int tiles;
+  int relu;
+  uint32_t plane, slab;          // bytes of one 8-channel plane (64 mod 128: the two planes' stores
+                                 // of one warp fall on different banks), of one slab
+  uint32_t stage;                // bytes from one stage to the next (slab, streamed weights)
+  int wres;                      // 1: the weights of every slice stay in shared memory
+  int cols;                      // tensor memory columns of one accumulator
+  int alloc;                     // columns allocated (a power of two)
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool in) {
+  const int n = in ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+
+// Weights of one slice: [P tap, x tap][channel half][R tap (descending), Cout] x 16 bytes.
 template <int COUT>
-__global__ void __launch_bounds__(TC_M) conv_fwd_tc_kernel(const bf16* __restrict__ in, const bf16* __restrict__ w,
-                                                           const float* __restrict__ bias, bf16* __restrict__ out,
-                                                           const Geo g, const int cin, const int relu,
-                                                           const long long voxels, int* err) {
-  constexpr int NCOL = COUT <= 32 ? 32 : (COUT <= 64 ? 64 : 128);  // TMEM columns: a power of two >= 32
-  constexpr uint32_t A_LBO = TC_M * 16, B_LBO = COUT * 16;          // bytes per K half
-  __shared__ __align__(128) uint8_t sA[2][2 * A_LBO];
-  __shared__ __align__(128) uint8_t sB[2][2 * B_LBO];
+__device__ __forceinline__ void halo_load_weights(uint32_t dst, const bf16* __restrict__ w, const HaloArgs& a, int kc,
+                                                  int tid) {
+  for (int i = tid; i < 27 * COUT * 2; i += HT_LOADERS) {
+    const int half = i & 1, co = (i >> 1) % COUT, t = (i >> 1) / COUT;  // t = (p * 3 + r) * 3 + x
+    const int x = t % 3, r = (t / 3) % 3, p = t / 9;
+    const int tap = p * a.tap_p + r * a.tap_r + x;
+    const bf16* src = w + ((long long)tap * COUT + co) * a.cin + kc * 16 + half * 8;
+    cp_async16(dst + (p * 3 + x) * (96 * COUT) + half * (48 * COUT) + ((2 - r) * COUT + co) * 16, src, true);
+  }
+}
+
+template <int BX>
+__device__ __forceinline__ void halo_load_slab(uint32_t dst, const bf16* __restrict__ in, const HaloArgs& a, int tile,
+                                               int kc, int tid) {
+  constexpr int PX = BX + 2, PP = HT_P + 2;
+  int t = tile;
+  const int x0 = (t % a.tx) * BX - 1;
+  t /= a.tx;
+  const int p0 = (t % a.tp) * HT_P - 1;
+  t /= a.tp;
+  const int r0 = (t % a.tr) * a.br - 1;
+  const int n = t / a.tr;
+  // Thread pairs take the two halves of a voxel (32 contiguous bytes); a thread's voxels lie
+  // STEP apart, so its coordinates and source advance by constants and carries (a division
+  // per voxel made the loads the longest part of an iteration).
+  constexpr int STEP = HT_LOADERS / 2, DX = STEP % PX, DP = STEP / PX;
+  static_assert(DP + 1 < PP, "one carry per axis and step");
+  const int half = tid & 1;
+  int v = tid >> 1;
+  int x = v % PX, p = v / PX, r = 0;
+  if (p >= PP) {
+    p -= PP;
+    r++;
+  }
+  const bf16* base = in + (long long)n * a.sn * a.cin + kc * 16 + half * 8;
+  long long off = (r0 + r) * a.sr + (p0 + p) * a.sp + x0 + x;
+  const long long step = DX + DP * a.sp, carry_x = a.sp - PX, carry_p = a.sr - PP * a.sp;
+  dst += half * a.plane + v * 16;
+#pragma unroll 2
+  for (const int end = (a.br + 2) * PP * PX; v < end; v += STEP) {
+    const bool ok = (unsigned)(x0 + x) < (unsigned)a.w && (unsigned)(p0 + p) < (unsigned)a.np &&
+                    (unsigned)(r0 + r) < (unsigned)a.nr;
+    cp_async16(dst, base + (ok ? off * a.cin : 0), ok);
+    dst += STEP * 16;
+    off += step;
+    x += DX;
+    p += DP;
+    if (x >= PX) {
+      x -= PX;
+      p++;
+      off += carry_x;
+    }
+    if (p >= PP) {
+      p -= PP;
+      r++;
+      off += carry_p;
+    }
+  }
+}
+
+template <int COUT, int BX>
+__global__ void __launch_bounds__(HT_THREADS, 1)
+    conv_halo_kernel(const bf16* __restrict__ in, const bf16* __restrict__ w, const float* __restrict__ bias,
+                     bf16* __restrict__ out, const HaloArgs a, int* err) {
+  constexpr int PX = BX + 2, PP = HT_P + 2, GX = BX / 8;
+  constexpr int NJ = 256 / COUT < 3 ? 256 / COUT : 3;  // output planes one MMA can take (N <= 256)
+  constexpr uint32_t WSLICE = 27 * COUT * 32;
+  extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ uint32_t tmem_base;
-  const int tid = threadIdx.x, warp = tid >> 5;
-  if (warp == 0) {
+  __shared__ float sbias[COUT];
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const uint32_t s0 = smem_addr(smem);
+  const uint32_t wbase = s0 + 2 * a.stage;  // resident weights follow the stages
+  if (warp == 8) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base)),
-                 "r"(NCOL)
+                 "r"(a.alloc)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -233,117 +348,163 @@ __global__ void __launch_bounds__(TC_M) conv_fwd_tc_kernel(const bf16* __restric
     tc_mbar_init(&bar[1]);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  for (int c = tid; c < COUT; c += HT_THREADS) sbias[c] = bias ? bias[c] : 0.f;
+  const int first = blockIdx.x, stride = gridDim.x;
+  const int mine = (a.tiles - first + stride - 1) / stride;
+  const int total = mine * a.kcs;
+  if (warp < 8) {
+    if (a.wres)
+      for (int k = 0; k < a.kcs; k++) halo_load_weights<COUT>(wbase + k * WSLICE, w, a, k, tid);
+    else
+      halo_load_weights<COUT>(s0 + a.slab, w, a, 0, tid);
+    halo_load_slab<BX>(s0, in, a, first, 0, tid);
+  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base;
+  const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+  const auto zero_cols = [&](uint32_t taddr) {  // 16 columns
+    const uint32_t z = 0u;
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+        "%1};" ::"r"(taddr),
+        "r"(z)
+        : "memory");
+  };
+  if (warp < 8) {  // every MMA accumulates: both accumulators start from zero
+    for (int c = (warp >> 2) * 16; c < 2 * a.cols; c += 32) zero_cols(tmem + lane_off + c);
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  }
 
-  // this thread's voxel: row `tid` of the A tile and lane `tid` of the accumulator
-  const long long v = (long long)blockIdx.x * TC_M + tid;
-  const bool valid = v < voxels;
-  long long t = valid ? v : 0;
-  const int x = (int)(t % g.w);
-  t /= g.w;
-  const int y = (int)(t % g.h);
-  t /= g.h;
-  const int z = (int)(t % g.d);
-  const uint32_t a_row = (uint32_t)((tid & 7) * 16 + (tid >> 3) * 128);
-  const int kcs = cin / 16, iters = 27 * kcs;
-  constexpr uint32_t IDESC = umma_idesc_bf16(TC_M, COUT);
-  uint32_t parity[2] = {0u, 0u};
+  // accumulator -> bias, ReLU, BF16 -> global, accumulator zeroed for its next tile
+  const auto epilogue = [&](int seq) {
+    int t = first + seq * stride;
+    const int x0 = (t % a.tx) * BX;
+    t /= a.tx;
+    const int p = (t % a.tp) * HT_P + (warp & 3) * 4 + (lane >> 3);
+    t /= a.tp;
+    const int r0 = (t % a.tr) * a.br;
+    const long long vox = (long long)(t / a.tr) * a.sn + p * a.sp + x0 + (lane & 7);
+    const uint32_t acc = tmem + lane_off + (uint32_t)((seq & 1) * a.cols);
+    for (int u = warp >> 2; u < GX * a.br; u += 2) {
+      const int g = u / a.br, r = r0 + u - g * a.br;
+      bf16* o = out + (vox + g * 8 + r * a.sr) * COUT;
+      const bool in_box = p < a.np && r < a.nr;
+#pragma unroll
+      for (int c0 = 0; c0 < COUT; c0 += 16) {
+        uint32_t q[16];
+        const uint32_t ta = acc + (uint32_t)(u * COUT + c0);
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+            "%15}, [%16];"
+            : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]),
+              "=r"(q[8]), "=r"(q[9]), "=r"(q[10]), "=r"(q[11]), "=r"(q[12]), "=r"(q[13]), "=r"(q[14]), "=r"(q[15])
+            : "r"(ta));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        zero_cols(ta);
+        if (in_box) {
+          float f[16];
+#pragma unroll
+          for (int k = 0; k < 16; k++) {
+            f[k] = __uint_as_float(q[k]) + sbias[c0 + k];
+            if (a.relu) f[k] = fmaxf(f[k], 0.f);
+          }
+#pragma unroll
+          for (int k = 0; k < 16; k += 8)
+            *reinterpret_cast<uint4*>(o + c0 + k) = make_uint4(pack_bf16(f[k], f[k + 1]), pack_bf16(f[k + 2], f[k + 3]),
+                                                               pack_bf16(f[k + 4], f[k + 5]), pack_bf16(f[k + 6], f[k + 7]));
+        }
+      }
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  };
+
   bool ok = true;
-  int issued = 0;
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  for (int it = 0; it < iters; it++) {
-    const int s = it & 1;
-    bool waited = true;
-    if (it >= 2) {  // the MMA of iteration it-2 read this stage
-      waited = tc_mbar_wait(&bar[s], parity[s]);
-      parity[s] ^= 1u;
+  int it = 0, seq = 0, kc = 0;  // iteration, tile (in this block's order) and slice
+  for (; it < total; it++) {
+    if (warp < 8) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads through the async proxy
     }
-    const int tap = it / kcs, kc = it - tap * kcs;
-    const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-    uint4 a0 = zero, a1 = zero;
-    const int xx = x + dx, yy = y + dy, zz = z + dz;
-    if (valid && xx >= 0 && xx < g.w && yy >= 0 && yy < g.h && zz >= 0 && zz < g.d) {
-      const long long nb = v + dx + (long long)g.w * (dy + (long long)g.h * dz);
-      const uint4* src = reinterpret_cast<const uint4*>(in + nb * cin + kc * 16);
-      a0 = __ldg(src);
-      a1 = __ldg(src + 1);
-    }
-    *reinterpret_cast<uint4*>(sA[s] + a_row) = a0;
-    *reinterpret_cast<uint4*>(sA[s] + A_LBO + a_row) = a1;
-    for (int r = tid; r < COUT * 2; r += TC_M) {
-      const int co = r >> 1, kh = r & 1;
-      const uint4 val = __ldg(reinterpret_cast<const uint4*>(w + ((long long)tap * COUT + co) * cin + kc * 16 + kh * 8));
-      *reinterpret_cast<uint4*>(sB[s] + kh * B_LBO + (co & 7) * 16 + (co >> 3) * 128) = val;
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads through the async proxy
-    if (!__syncthreads_and(waited)) {  // a wait gave up somewhere: stop issuing (block-uniform)
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (!__syncthreads_and(ok)) {  // a wait gave up: stop issuing (block-uniform)
       ok = false;
       break;
     }
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint64_t adesc = umma_desc(smem_addr(sA[s]), A_LBO, 128);
-      const uint64_t bdesc = umma_desc(smem_addr(sB[s]), B_LBO, 128);
-      const uint32_t acc = it > 0 ? 1u : 0u, mask0 = 0u;
-      asm volatile(
-          "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-          " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n" ::"r"(tmem),
-          "l"(adesc), "l"(bdesc), "r"(IDESC), "r"(acc), "r"(mask0)
-          : "memory");
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                       smem_addr(&bar[s]))
-                   : "memory");
-    }
-    issued = it + 1;
-  }
-  // the last commit tracks every MMA issued before it
-  bool done = true;
-  if (issued > 0) done = tc_mbar_wait(&bar[(issued - 1) & 1], parity[(issued - 1) & 1]);
-  ok = __syncthreads_and(ok && done) != 0;
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (ok && valid) {
-    uint32_t* o32 = reinterpret_cast<uint32_t*>(out + v * COUT);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t slab = s0 + (it & 1) * a.stage;
+    if (warp == 8) {
+      if (elect_one()) {
+        const uint32_t wt = a.wres ? wbase + kc * WSLICE : slab + a.slab;
+        const uint32_t acc = tmem + (uint32_t)((seq & 1) * a.cols);
+        const int r0 = ((first + seq * stride) / (a.tx * a.tp) % a.tr) * a.br;
+        const int rout = a.nr - r0 < a.br ? a.nr - r0 : a.br;  // output planes inside the box
+        const uint64_t alo = umma_desc(0, a.plane, PX * 16), blo = umma_desc(0, 48 * COUT, 128);
+        for (int r = 0; r < rout + 2; r++) {
+          if (r0 + r - 1 < 0 || r0 + r - 1 >= a.nr) continue;  // an input plane outside the box is zero
+          const int j1 = rout + 1 - r < 2 ? rout + 1 - r : 2;
+          for (int j0 = r < 2 ? 2 - r : 0; j0 <= j1; j0 += NJ) {
+            const int nj = j1 - j0 + 1 < NJ ? j1 - j0 + 1 : NJ;
+            const uint32_t idesc = umma_idesc_bf16(TC_M, nj * COUT);
+            for (int g = 0; g < GX; g++) {
+              const uint32_t d = acc + (uint32_t)((g * a.br + r - 2 + j0) * COUT);
+              // start addresses in 16-byte units; they stay below 2^14 for every tap
+              const uint64_t ad = alo | ((slab >> 4) + r * PP * PX + g * 8), bd = blo | ((wt >> 4) + j0 * COUT);
 #pragma unroll
-    for (int c0 = 0; c0 < COUT; c0 += 8) {
-      uint32_t r[8];
-      asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                   : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                   : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      float f[8];
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        f[k] = __uint_as_float(r[k]) + (bias ? bias[c0 + k] : 0.f);
-        if (relu) f[k] = fmaxf(f[k], 0.f);
+              for (int px = 0; px < 9; px++)
+                asm volatile(
+                    "{\n .reg .pred p;\n setp.ne.b32 p, 1, 0;\n"
+                    " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+                    "l"(ad + px / 3 * PX + px % 3), "l"(bd + px * (6 * COUT)), "r"(idesc)
+                    : "memory");
+            }
+          }
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                         smem_addr(&bar[it & 1]))
+                     : "memory");
       }
-      const uint4 packed = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
-                                      pack_bf16(f[6], f[7]));
-      *reinterpret_cast<uint4*>(o32 + c0 / 2) = packed;
+      __syncwarp();
+    } else {
+      if (it > 0) {  // the MMAs of the previous iteration: they read the other stage
+        ok = __all_sync(0xffffffffu, tc_mbar_wait(&bar[(it - 1) & 1], (uint32_t)(((it - 1) >> 1) & 1)));
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
+      if (ok && it + 1 < total) {
+        const int nk = kc + 1 == a.kcs ? 0 : kc + 1, ns = nk ? seq : seq + 1;
+        const uint32_t next = s0 + ((it + 1) & 1) * a.stage;
+        if (!a.wres) halo_load_weights<COUT>(next + a.slab, w, a, nk, tid);
+        halo_load_slab<BX>(next, in, a, first + ns * stride, nk, tid);
+      }
+      if (ok && kc == 0 && seq > 0) epilogue(seq - 1);
     }
-  } else if (ok) {
-    // lanes past the last voxel still take part in the warp-wide loads
-#pragma unroll
-    for (int c0 = 0; c0 < COUT; c0 += 8) {
-      uint32_t r[8];
-      asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                   : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                   : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    if (++kc == a.kcs) {
+      kc = 0;
+      seq++;
     }
   }
-  if (!ok && tid == 0) atomicExch(err, 1);
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  // the last commit tracks every MMA before it
+  if (it > 0) {
+    const bool done = tc_mbar_wait(&bar[(it - 1) & 1], (uint32_t)(((it - 1) >> 1) & 1));
+    ok = ok && done;
+  }
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (__syncthreads_and(ok)) {
+    if (warp < 8) epilogue(mine - 1);
+  } else if (tid == 0) {
+    atomicExch(err, 1);
+  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NCOL) : "memory");
+  if (warp == 8)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.alloc) : "memory");
 }
 
 // ---- tcgen05 convolution fed by TMA --------------------------------------------------
-// Same tiling as conv_fwd_tc_kernel, but the A tile of a tap is a TMA box of the
-// activations: a 5-D tensor map over (C, W, H, D, N) with box {8, min(W,128),
+// A CTA owns 128 consecutive voxels (M = 128) and all output channels (N = Cout); the A tile
+// of a tap is a TMA box of the activations: a 5-D tensor map over (C, W, H, D, N) with box {8, min(W,128),
 // 128 / min(W,128), 1, 1} lands in shared memory as 128 rows of 16 bytes — exactly the
 // K-major interleaved core-matrix layout (8-row groups 128 bytes apart) — and its
 // out-of-range rows (the 1-voxel halo at the box faces) are filled with zeros by the
@@ -838,11 +999,9 @@ __global__ void unpack_fields_kernel(const bf16* __restrict__ y, float* __restri
   }
 }
 
-// forward convolutions: 0 = mma.sync warp tiles, 1 = tcgen05 with thread-gathered tiles,
-// 2 = per layer (tcgen05 when Cout >= 32: with Cout = 16 one 128-voxel gather feeds too
-// small an MMA and the warp tiles are faster, measured on B200), 3 = tcgen05 with
-// TMA-fed tiles where the shape allows (slower on B200 with these 16-byte-wide boxes:
-// the copy engine issues one request per 16-byte row)
+// forward convolutions: 0 = mma.sync warp tiles, 1 and 2 = halo tiles, 3 = tcgen05 with one
+// TMA box per tap where the shape allows (slower on B200 with these 16-byte-wide boxes: the
+// copy engine issues one request per 16-byte row, and 27 times per voxel)
 int g_engine = 2;
 
 // cuTensorMapEncodeTiled from the driver (fetched once, no link against libcuda).
@@ -885,6 +1044,117 @@ int* tc_err_ptr() {
 
 unsigned blocks_for(long long count, int per) { return (unsigned)((count + per - 1) / per); }
 
+bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
+
+int sm_count() {
+  static std::atomic<int> counts[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  int c = counts[dev].load(std::memory_order_relaxed);
+  if (!c) {
+    if (cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || c <= 0) c = 148;
+    counts[dev].store(c, std::memory_order_relaxed);
+  }
+  return c;
+}
+
+// Raises a kernel's dynamic shared memory limit once per device.
+template <class K>
+bool allow_smem(K kernel, int bytes, std::atomic<unsigned long long>& done) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  if ((done.load(std::memory_order_acquire) >> dev) & 1ull) return true;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+  done.fetch_or(1ull << dev, std::memory_order_release);
+  return true;
+}
+
+// Tile of a halo convolution: x width (8 or 16), planes along R, which axis is P.  The
+// model counts cycles of the longest block: MMAs (33 + N / 4 cycles of operand reads or N / 2
+// of arithmetic, measured on B200) against staged bytes, and the fixed cost of an iteration.
+struct HaloPlan {
+  HaloArgs a;
+  int bx;
+  unsigned grid;
+  uint32_t smem;
+};
+
+bool halo_plan(const Geo& g, int cin, int cout, int sms, HaloPlan& best) {
+  const int kcs = cin / 16, nj = 256 / cout < 3 ? 256 / cout : 3;
+  const uint32_t wslice = 27u * cout * 32u;
+  double best_cost = 1e300;
+  for (int bx = 8; bx <= 16; bx += 8)
+    for (int swap = 0; swap < 2; swap++)
+      for (int br = 1; 2 * (bx / 8) * br * cout <= 512; br++) {
+        HaloArgs a{};
+        a.n = g.n;
+        a.w = g.w;
+        a.np = swap ? g.d : g.h;
+        a.nr = swap ? g.h : g.d;
+        const long long sy = g.w, sz = (long long)g.w * g.h;
+        a.sp = swap ? sz : sy;
+        a.sr = swap ? sy : sz;
+        a.sn = sz * g.d;
+        a.tap_p = swap ? 9 : 3;
+        a.tap_r = swap ? 3 : 9;
+        a.cin = cin;
+        a.kcs = kcs;
+        a.br = br;
+        a.tx = g.w / bx;
+        a.tp = (a.np + HT_P - 1) / HT_P;
+        a.tr = (a.nr + br - 1) / br;
+        const long long tiles = (long long)a.tx * a.tp * a.tr * a.n;
+        if (tiles > 0x7fffffffLL / (kcs + 1)) continue;
+        a.tiles = (int)tiles;
+        const uint32_t raw = (uint32_t)(br + 2) * (HT_P + 2) * (bx + 2) * 16u;
+        a.plane = raw + (192u - raw % 128u) % 128u;
+        a.slab = 2 * a.plane;
+        a.wres = 2 * a.slab + kcs * wslice <= (uint32_t)HT_MAX_SMEM;
+        a.stage = a.slab + (a.wres ? 0u : wslice);
+        const uint32_t smem = 2 * a.stage + (a.wres ? kcs * wslice : 0u);
+        if (smem > (uint32_t)HT_MAX_SMEM) break;
+        a.cols = (bx / 8) * br * cout;
+        a.alloc = 32;
+        while (a.alloc < 2 * a.cols) a.alloc *= 2;
+        double mma = 0;
+        for (int r = 0; r < br + 2; r++)
+          for (int j0 = r < 2 ? 2 - r : 0, j1 = br + 1 - r < 2 ? br + 1 - r : 2; j0 <= j1; j0 += nj) {
+            const int n = (j1 - j0 + 1 < nj ? j1 - j0 + 1 : nj) * cout;
+            mma += 9.0 * (bx / 8) * (n / 2 > 33 + n / 4 ? n / 2 : 33 + n / 4);
+          }
+        const double load = a.stage / 24.0;
+        const double cost = (double)((tiles + sms - 1) / sms) * kcs * ((mma > load ? mma : load) + 800.0) +
+                            (a.wres ? kcs * wslice / 24.0 : 0.0);
+        if (cost < best_cost) {
+          best_cost = cost;
+          best.a = a;
+          best.bx = bx;
+          best.grid = (unsigned)(tiles < sms ? tiles : sms);
+          best.smem = smem;
+        }
+      }
+  return best_cost < 1e300;
+}
+
+template <int COUT, int BX>
+int halo_launch(const bf16* in, const bf16* w, const float* bias, bf16* out, const HaloPlan& p, int* err,
+                cudaStream_t s) {
+  static std::atomic<unsigned long long> done{0};
+  if (!allow_smem(conv_halo_kernel<COUT, BX>, HT_MAX_SMEM, done)) return launched("nn_conv3d_fwd (shared memory)");
+  conv_halo_kernel<COUT, BX><<<p.grid, HT_THREADS, p.smem, s>>>(in, w, bias, out, p.a, err);
+  return launched("nn_conv3d_fwd (tcgen05)");
+}
+
+template <int COUT>
+int halo_conv(const bf16* in, const bf16* w, const float* bias, bf16* out, const Geo& g, int cin, int relu, int* err,
+              cudaStream_t s) {
+  HaloPlan p{};
+  if (!halo_plan(g, cin, COUT, sm_count(), p)) return fail("nn_conv3d_fwd: no tile for %d x %d x %d", g.d, g.h, g.w);
+  p.a.relu = relu;
+  return p.bx == 16 ? halo_launch<COUT, 16>(in, w, bias, out, p, err, s)
+                    : halo_launch<COUT, 8>(in, w, bias, out, p, err, s);
+}
+
 bool geo_ok(int n, int d, int h, int w) { return n > 0 && d > 0 && h > 0 && w > 0; }
 
 }  // namespace
@@ -906,7 +1176,7 @@ int32_t nn_conv3d_fwd(const void* in, const void* w, const float* bias, void* ou
   const bf16* I = (const bf16*)in;
   const bf16* W = (const bf16*)w;
   bf16* O = (bf16*)out;
-  if (g_engine == 1 || g_engine == 3 || (g_engine == 2 && cout >= 32)) {
+  if (g_engine != 0) {
     int* err = tc_err_ptr();
     if (!err) return fail("nn_conv3d_fwd: no device address for the error word");
     PFN_cuTensorMapEncodeTiled_v12000 enc = g_engine == 3 ? tensor_map_encoder() : nullptr;
@@ -939,17 +1209,16 @@ int32_t nn_conv3d_fwd(const void* in, const void* w, const float* bias, void* ou
       }
       return launched("nn_conv3d_fwd (tcgen05, TMA)");
     }
-    const long long vox = (long long)n * d * h * wd;
-    const unsigned tgrid = blocks_for(vox, TC_M);
-    switch (cout) {
-      case 16: conv_fwd_tc_kernel<16><<<tgrid, TC_M, 0, s>>>(I, W, bias, O, g, cin, relu, vox, err); break;
-      case 32: conv_fwd_tc_kernel<32><<<tgrid, TC_M, 0, s>>>(I, W, bias, O, g, cin, relu, vox, err); break;
-      case 48: conv_fwd_tc_kernel<48><<<tgrid, TC_M, 0, s>>>(I, W, bias, O, g, cin, relu, vox, err); break;
-      case 64: conv_fwd_tc_kernel<64><<<tgrid, TC_M, 0, s>>>(I, W, bias, O, g, cin, relu, vox, err); break;
-      case 96: conv_fwd_tc_kernel<96><<<tgrid, TC_M, 0, s>>>(I, W, bias, O, g, cin, relu, vox, err); break;
-      default: return fail("nn_conv3d_fwd: Cout %d not in {16, 32, 48, 64, 96}", cout);
+    if (aligned16(in) && aligned16(w) && aligned16(out)) {
+      switch (cout) {
+        case 16: return halo_conv<16>(I, W, bias, O, g, cin, relu, err, s);
+        case 32: return halo_conv<32>(I, W, bias, O, g, cin, relu, err, s);
+        case 48: return halo_conv<48>(I, W, bias, O, g, cin, relu, err, s);
+        case 64: return halo_conv<64>(I, W, bias, O, g, cin, relu, err, s);
+        case 96: return halo_conv<96>(I, W, bias, O, g, cin, relu, err, s);
+        default: return fail("nn_conv3d_fwd: Cout %d not in {16, 32, 48, 64, 96}", cout);
+      }
     }
-    return launched("nn_conv3d_fwd (tcgen05)");
   }
   switch (cout) {
     case 16: conv_fwd_kernel<2><<<grid, 128, 0, s>>>(I, W, bias, O, g, cin, relu, tiles); break;

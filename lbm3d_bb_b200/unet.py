@@ -83,8 +83,8 @@ ENGINES = {"mma": 0, "tcgen05": 1, "auto": 2, "tcgen05-tma": 3}
 
 
 def set_conv_engine(name: str) -> str:
-    """Selects the forward-convolution kernels ('mma', 'tcgen05', 'auto': tcgen05 for
-    Cout >= 32, or 'tcgen05-tma'); returns the previous one."""
+    """Selects the forward-convolution kernels ('mma': warp tiles, 'tcgen05' and 'auto': halo
+    tiles on tcgen05, or 'tcgen05-tma'); returns the previous one."""
     prev = lib().nn_set_conv_engine(ENGINES[name])
     if prev not in (0, 1, 2, 3):
         raise NnError((lib().nn_last_error() or b"").decode(errors="replace"))
