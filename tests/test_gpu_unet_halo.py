@@ -71,3 +71,27 @@ def test_halo_conv_without_bias(gpu):
 def test_unaligned_input_takes_the_warp_tiles(gpu, cout):
     got, ref = _run((1, 4, 5, 32), 16, cout, relu=True, shift=2)  # 4-byte aligned only
     assert rel_l2(got, ref) <= TOL
+
+
+@pytest.mark.parametrize("shape,cin,cout", [
+    ((1, 1, 1, 16), 16, 16),     # one voxel row: every tap but the x ones outside
+    ((1, 2, 3, 20), 16, 32),     # x not a multiple of the 16-voxel K step
+    ((2, 5, 17, 32), 32, 32),    # planes of two samples side by side, y past a tile
+    ((1, 9, 4, 48), 48, 16),     # three input slices
+    ((1, 17, 6, 16), 96, 64),    # several input slices and output blocks
+    ((3, 40, 37, 64), 16, 16),   # several tiles per block, z and y remainders
+    ((2, 24, 40, 64), 64, 64),
+])
+def test_weight_gradient_tiles(gpu, shape, cin, cout):
+    """FP32 sums of exact BF16 products, added onto what dw holds (tolerance of the layer tests)."""
+    import torch
+
+    rng = np.random.default_rng(sum(shape) + cin + cout)
+    x = U.to_bf16(rng.standard_normal(shape + (cin,)))
+    dy = U.to_bf16(rng.standard_normal(shape + (cout,)))
+    start = rng.standard_normal((27, cout, cin)).astype(np.float32)
+    _, ref, _ = U.conv_bwd(x, np.zeros((27, cout, cin)), dy)
+    dw = torch.from_numpy(start).cuda()
+    N.Ops().bwd_weight(_bf16(x), _bf16(dy), dw, shape, cin, cout)
+    N.tc_status()
+    assert rel_l2(dw.cpu().numpy(), start + ref) <= 1e-5
