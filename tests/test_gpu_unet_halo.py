@@ -95,3 +95,72 @@ def test_weight_gradient_tiles(gpu, shape, cin, cout):
     N.Ops().bwd_weight(_bf16(x), _bf16(dy), dw, shape, cin, cout)
     N.tc_status()
     assert rel_l2(dw.cpu().numpy(), start + ref) <= 1e-5
+
+
+@pytest.mark.parametrize("c", [16, 32, 48, 4])
+@pytest.mark.parametrize("shift", [0, 2])
+def test_elementwise_forms(gpu, c, shift):
+    """Grouped and one-element forms of the elementwise kernels (4 channels and misaligned
+    tensors take the latter) on a box with a ragged row: copies and maxima exactly, sums to the
+    BF16 rounding of the stored result (2^-9) or FP32 summation (1e-5)."""
+    import torch
+
+    ops = N.Ops()
+    shape = (3, 2, 4, 22)
+    coarse = (3, 1, 2, 11)
+    rng = np.random.default_rng(c + shift)
+
+    def dev(a):
+        flat = torch.zeros(a.size + 8, dtype=torch.bfloat16, device="cuda")
+        t = flat[shift:shift + a.size].view(a.shape)
+        t.copy_(_bf16(a))
+        return t
+
+    def host(t):
+        return t.float().cpu().numpy().astype(np.float64)
+
+    x, y, dp = (U.to_bf16(rng.standard_normal(s + (c,))) for s in (shape, shape, coarse))
+    p = dev(np.zeros(coarse + (c,)))
+    ops.pool(dev(x), p, shape, c)
+    assert rel_l2(host(p), U.pool(x)) <= 2.0 ** -8
+    for acc in (False, True):
+        g = dev(x)
+        ops.pool_bwd(dev(dp), g, shape, c, acc)
+        assert rel_l2(host(g), U.pool_bwd(dp) + (x if acc else 0)) <= 2.0 ** -8
+    cat = dev(np.zeros(shape + (2 * c,)))
+    ops.up_cat(dev(dp), dev(x), cat, shape, c, c)
+    assert np.array_equal(host(cat), np.concatenate([U.up(dp), x], axis=-1))
+    dcat = np.concatenate([y, x], axis=-1)
+    dlow, dskip = dev(np.zeros(coarse + (c,))), dev(np.zeros(shape + (c,)))
+    ops.up_cat_bwd(dev(dcat), dlow, dskip, shape, c, c)
+    assert rel_l2(host(dlow), U.up_bwd(y)) <= 2.0 ** -8
+    assert np.array_equal(host(dskip), x)
+    g = dev(x)
+    ops.relu_bwd(g, dev(y))
+    assert np.array_equal(host(g), x * (y > 0))
+    db = torch.ones(c, device="cuda")
+    ops.bias_grad(dev(x), db, int(np.prod(shape)), c)
+    assert rel_l2(host(db), 1 + x.reshape(-1, c).sum(0)) <= 1e-5
+
+
+@pytest.mark.parametrize("cpad,ct", [(16, 4), (16, 3), (8, 4)])
+def test_masked_loss_forms(gpu, cpad, ct):
+    import torch
+
+    vox = 70001  # a ragged last block, several voxels per thread of the grid at most
+    rng = np.random.default_rng(cpad + ct)
+    out, t = U.to_bf16(rng.standard_normal((vox, cpad))), rng.standard_normal((vox, ct)).astype(np.float32)
+    mask, cw = (rng.random(vox) > 0.3).astype(np.uint8), (0.5 + rng.random(ct)).astype(np.float32)
+    count = float(mask.sum())
+    od = _bf16(out)
+    dout = torch.full((vox, cpad), 7.0, dtype=torch.bfloat16, device="cuda")
+    loss = torch.ones(1, dtype=torch.float64, device="cuda")
+    L, dev = N.lib(), lambda a: torch.from_numpy(a).cuda()
+    td, md, cd = dev(t), dev(mask), dev(cw)
+    assert L.nn_mse(od.data_ptr(), td.data_ptr(), md.data_ptr(), cd.data_ptr(), dout.data_ptr(), loss.data_ptr(), vox,
+                    cpad, ct, count, None) == 0
+    d = (out[:, :ct].astype(np.float32) - t).astype(np.float64) * mask[:, None]
+    ref = np.zeros((vox, cpad))
+    ref[:, :ct] = 2 * cw * d / count
+    assert abs(float(loss) - 1 - (cw * d * d).sum() / count) <= 1e-12 * vox
+    assert rel_l2(dout.float().cpu().numpy(), ref) <= 2.0 ** -8
