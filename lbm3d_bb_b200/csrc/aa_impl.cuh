@@ -402,20 +402,17 @@ __device__ __noinline__ void aa_general(const AAParams& p, typename SP::S* __res
   const bool on_face = (xs0 | xs2 | ys0 | ys2 | zs0 | zs2) < 0;
   const bool near = (fl & F_NEAR) != 0;
 
+  // the link word holds what the flags of the 18 neighbours say (near_kernel): one load
+  // instead of 18 bytes at scattered addresses
   uint32_t face = 0, bcp = 0, bcc = 0, mov = 0;
-  if (on_face || near) {
-#pragma unroll
-    for (int d = 0; d < 18; d++) {
-      const int sx = xs[1 - cx(d)], sy = ys[1 - cy(d)], sz = zs[1 - cz(d)];
-      if ((sx | sy | sz) < 0) {
-        face |= 1u << d;
-      } else if (near) {
-        const uint8_t fs = flags[sx + nxl * sy + nxy * sz];
-        if (fs & F_SOLID_PREV) bcp |= 1u << d;
-        if (fs & F_SOLID) bcc |= 1u << d;
-        if (fs & F_MOVING) mov |= 1u << d;
-      }
-    }
+  if (on_face)
+    face = (xs0 < 0 ? dir_mask(0, 1) : 0u) | (xs2 < 0 ? dir_mask(0, -1) : 0u) | (ys0 < 0 ? dir_mask(1, 1) : 0u) |
+           (ys2 < 0 ? dir_mask(1, -1) : 0u) | (zs0 < 0 ? dir_mask(2, 1) : 0u) | (zs2 < 0 ? dir_mask(2, -1) : 0u);
+  if (near) {
+    const unsigned long long lw = p.links[i];
+    bcc = (uint32_t)(lw & 0x3FFFFu) & ~face;
+    bcp = (uint32_t)((lw >> 18) & 0x3FFFFu) & ~face;
+    mov = (uint32_t)((lw >> 36) & 0x3FFFFu) & ~face;
   }
   const uint32_t bcr = face | bcp;  // incoming slots holding boundary values (read side)
   const uint32_t bcw = face | bcc;  // incoming slots to fill with boundary values (write side)
@@ -824,18 +821,45 @@ struct Pair2<double> {
 };
 
 template <class SP, bool ODD, bool TRT, int FORCE>
-__device__ __forceinline__ void pair_cell(const AAParams& p, const typename SP::C* f, typename SP::C* pst) {
+__device__ __forceinline__ void pair_cell(const AAParams& p, const typename SP::C* f, typename SP::C* pst,
+                                          typename SP::C& rho, typename SP::C& ux, typename SP::C& uy,
+                                          typename SP::C& uz) {
   using C = typename SP::C;
   const Coll<C> k{C(p.omega_p), C(p.omega_m), C(p.gacc[0]), C(p.gacc[1]), C(p.gacc[2])};
   const C rho0 = C(p.rho0);
-  C rho, ux, uy, uz;
   moments<C, FORCE, SP::DEV>(f, k, rho, ux, uy, uz, rho0);
   collide<C, TRT, FORCE, SP::DEV>(f, pst, k, rho, ux, uy, uz, rho0);
 }
+template <class SP, bool ODD, bool TRT, int FORCE>
+__device__ __forceinline__ void pair_cell(const AAParams& p, const typename SP::C* f, typename SP::C* pst) {
+  typename SP::C rho, ux, uy, uz;
+  pair_cell<SP, ODD, TRT, FORCE>(p, f, pst, rho, ux, uy, uz);
+}
+
+// The same for a cell on a non-periodic x face (SIGN: incoming directions with c_x = SIGN come
+// from outside when on_face): the outgoing populations opp(d) of those directions, which leave
+// the box, are replaced by the face values of d, so that the store of opp(d), kept in the own
+// slot d, stores the boundary value.
+template <class SP, bool ODD, bool TRT, int FORCE, bool FACES, int SIGN>
+__device__ __forceinline__ void pair_cell_x(const AAParams& p, const typename SP::C* f, typename SP::C* pst,
+                                            const bool on_face) {
+  using C = typename SP::C;
+  C rho, ux, uy, uz;
+  pair_cell<SP, ODD, TRT, FORCE>(p, f, pst, rho, ux, uy, uz);
+  if (FACES && on_face) {
+#pragma unroll
+    for (int d = 0; d < 18; d++)
+      if (cx(d) == SIGN)
+        pst[opp(d)] = face_value<C>(p, d, SIGN > 0, SIGN < 0, false, false, rho, ux, uy, uz, pst,
+                                    SP::DEV ? wgt<C>(d) * C(p.rho0) : C(0));
+  }
+}
 
 // The update of the cell pair (x0, x0 + 1), x0 even, as described above; all 32 lanes of the
-// warp take part (warp vote).
-template <class SP, bool ODD, bool TRT, int FORCE>
+// warp take part (warp vote).  FACES: some axis is not periodic; a pair in a row off the y and z
+// faces is updated here, the cells of an x face included, and warps with a row on one of them
+// take the one-cell path for both cells.
+template <class SP, bool ODD, bool TRT, int FORCE, bool FACES = false>
 __device__ __forceinline__ void pair_cells(const AAParams& p, typename SP::S* __restrict__ A,
                                            const uint8_t* __restrict__ flags, const int x0, const int y, const int z,
                                            const bool inb, double* acc, bool& has_link) {
@@ -843,15 +867,28 @@ __device__ __forceinline__ void pair_cells(const AAParams& p, typename SP::S* __
   using C = typename SP::C;
   const Grid& g = p.g;
   const long long i0 = inb ? node_index(g, x0, y, z) : 0;
-  const bool coord_fast = inb && (!ODD || (y > 0 && y < g.ny - 1 && z > 0 && z < g.nz - 1));
+  const bool yz_inside = y > 0 && y < g.ny - 1 && z > 0 && z < g.nz - 1;
+  bool coord_fast = inb && (!ODD || yz_inside);
+  // cell 0 on the low x face, cell 1 on the high one
+  const bool xlo = FACES && !g.per[0] && x0 == 0, xhi = FACES && !g.per[0] && x0 + 1 == g.nx - 1;
+  if (FACES) {
+    if (!ODD)  // own slots only: a periodic axis has no special rows
+      coord_fast = inb && (g.per[1] || (y > 0 && y < g.ny - 1)) && (g.per[2] || (z > 0 && z < g.nz - 1));
+    if (!__all_sync(0xffffffffu, coord_fast || !inb)) {
+#pragma unroll 1
+      for (int h = 0; h < 2; h++)
+        aa_direct<SP, ODD, TRT, FORCE, true>(p, A, flags, x0 + h, y, z, inb, acc, &has_link);
+      return;
+    }
+  }
   uint32_t fl0 = F_SOLID, fl1 = F_SOLID;
   if (inb) {
     const uint32_t fw = *reinterpret_cast<const unsigned short*>(flags + i0);
     fl0 = fw & 0xFFu;
     fl1 = fw >> 8;
   }
-  const long long fix_lo = x0 == 0 ? (long long)g.nx : 0;            // cell 0 at x = 0
-  const long long fix_hi = x0 + 1 == g.nx - 1 ? (long long)g.nx : 0;  // cell 1 at x = nx - 1
+  const long long fix_lo = x0 == 0 && !xlo ? (long long)g.nx : 0;            // cell 0 at x = 0
+  const long long fix_hi = x0 + 1 == g.nx - 1 && !xhi ? (long long)g.nx : 0;  // cell 1 at x = nx - 1
   C f0[Q], f1[Q];
   // byte bases: the cell pair, and each cell with its periodic x wrap folded in; with the
   // byte offsets of the parameter block each access is one 64-bit add (FP32 on B200:
@@ -859,6 +896,8 @@ __device__ __forceinline__ void pair_cells(const AAParams& p, typename SP::S* __
   const char* const Bi = reinterpret_cast<const char*>(A + i0);
   const char* const B0 = reinterpret_cast<const char*>(A + i0 + fix_lo);
   const char* const B1 = reinterpret_cast<const char*>(A + i0 + 1 - fix_hi);
+  // own slot of direction d, where the boundary value of an x face lies
+  const auto own = [&](const int d) { return Bi + (long long)d * g.plane * (long long)sizeof(S); };
   if (coord_fast) {
 #pragma unroll
     for (int d = 0; d < Q; d++) {
@@ -866,11 +905,11 @@ __device__ __forceinline__ void pair_cells(const AAParams& p, typename SP::S* __
       if (!ODD || cx(d) == 0) {
         Pair2<S>::ld(reinterpret_cast<const S*>(Bi + o), f0[d], f1[d]);
       } else if (cx(d) == 1) {
-        f0[d] = ld_fast<SP>(reinterpret_cast<const S*>(B0 + o), d, C(p.rho0));
+        f0[d] = ld_fast<SP>(reinterpret_cast<const S*>(xlo ? own(d) : B0 + o), d, C(p.rho0));
         f1[d] = ld_fast<SP>(reinterpret_cast<const S*>(Bi + o) + 1, d, C(p.rho0));
       } else {
         f0[d] = ld_fast<SP>(reinterpret_cast<const S*>(Bi + o), d, C(p.rho0));
-        f1[d] = ld_fast<SP>(reinterpret_cast<const S*>(B1 + o), d, C(p.rho0));
+        f1[d] = ld_fast<SP>(reinterpret_cast<const S*>(xhi ? own(d) + sizeof(S) : B1 + o), d, C(p.rho0));
       }
     }
   }
@@ -900,13 +939,13 @@ __device__ __forceinline__ void pair_cells(const AAParams& p, typename SP::S* __
       }
       C p0[Q], p1[Q];
       if (!solid0) {
-        pair_cell<SP, ODD, TRT, FORCE>(p, f0, p0);
+        pair_cell_x<SP, ODD, TRT, FORCE, FACES, 1>(p, f0, p0, xlo);
       } else {
 #pragma unroll
         for (int d = 0; d < Q; d++) p0[d] = C(0);
       }
       if (!solid1) {
-        pair_cell<SP, ODD, TRT, FORCE>(p, f1, p1);
+        pair_cell_x<SP, ODD, TRT, FORCE, FACES, -1>(p, f1, p1, xhi);
       } else {
 #pragma unroll
         for (int d = 0; d < Q; d++) p1[d] = C(0);
@@ -924,9 +963,11 @@ __device__ __forceinline__ void pair_cells(const AAParams& p, typename SP::S* __
             Pair2<S>::st(reinterpret_cast<S*>(bi), p0[j], p1[j]);
           } else if (cx(j) == 1) {
             st_fast<SP>(reinterpret_cast<S*>(bi), p0[j], j, rho0);
-            st_fast<SP>(reinterpret_cast<S*>(const_cast<char*>(B1) + o), p1[j], j, rho0);
+            st_fast<SP>(reinterpret_cast<S*>(const_cast<char*>(xhi ? own(opp(j)) + sizeof(S) : B1 + o)), p1[j],
+                        xhi ? opp(j) : j, rho0);
           } else {
-            st_fast<SP>(reinterpret_cast<S*>(const_cast<char*>(B0) + o), p0[j], j, rho0);
+            st_fast<SP>(reinterpret_cast<S*>(const_cast<char*>(xlo ? own(opp(j)) : B0 + o)), p0[j], xlo ? opp(j) : j,
+                        rho0);
             st_fast<SP>(reinterpret_cast<S*>(bi) + 1, p1[j], j, rho0);
           }
         }
@@ -945,12 +986,12 @@ __device__ __forceinline__ void pair_cells(const AAParams& p, typename SP::S* __
           }
           if (!solid0) {
             long long a = i0 + o + (cx(j) == -1 ? fix_lo : 0);
-            if (j < 18 && ((bc0 >> oj) & 1u)) a = (long long)oj * g.plane + i0;
+            if (j < 18 && (((bc0 >> oj) & 1u) || (xlo && cx(j) == -1))) a = (long long)oj * g.plane + i0;
             st_fast<SP>(A + a, p0[j], j, rho0);
           }
           if (!solid1) {
             long long a = i0 + 1 + o - (cx(j) == 1 ? fix_hi : 0);
-            if (j < 18 && ((bc1 >> oj) & 1u)) a = (long long)oj * g.plane + i0 + 1;
+            if (j < 18 && (((bc1 >> oj) & 1u) || (xhi && cx(j) == 1))) a = (long long)oj * g.plane + i0 + 1;
             st_fast<SP>(A + a, p1[j], j, rho0);
           }
         }
@@ -967,8 +1008,20 @@ __device__ __forceinline__ void pair_cells(const AAParams& p, typename SP::S* __
   }
 }
 
+// Block shapes of the pair kernels (threads along x, rows) and blocks per SM.  Registers and
+// spills are those of 768 threads per SM (80 registers) or, for TRT in FP32, 640 (96); smaller
+// blocks start and end more evenly.  B200, us per step, blocks of 256 before: FP32 512^3 BGK
+// 3527 / 3415 (64 threads), 384x192x192 TRT 413 / 381; FP16 deviations 512^3 2299 / 2222 with
+// 128 threads in the split odd kernel and 64 in the even kernels (64 in the odd one too costs
+// 8 % of a step with forces: a reduction per block).
+constexpr int PAIR_X = 64, SPLIT_ROWS = 2, QUAD_ROWS = 2, OCTO_ROWS = 2;
+template <class SP, bool TRT>
+constexpr int pair_blocks() {
+  return SP::MIN_BLOCKS > 2 ? (TRT ? 10 : 12) : 4;
+}
+
 template <class SP, bool ODD, bool TRT, int FORCE>
-__global__ void __launch_bounds__(256, (SP::MIN_BLOCKS > 2 ? 3 : 1)) aa_pair_kernel(const __grid_constant__ AAParams p,
+__global__ void __launch_bounds__(PAIR_X, pair_blocks<SP, TRT>()) aa_pair_kernel(const __grid_constant__ AAParams p,
                                                                                 typename SP::S* __restrict__ A,
                                                                                 const uint8_t* __restrict__ flags) {
   const Grid& g = p.g;
@@ -981,6 +1034,33 @@ __global__ void __launch_bounds__(256, (SP::MIN_BLOCKS > 2 ? 3 : 1)) aa_pair_ker
   double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   bool has_link = false;
   pair_cells<SP, ODD, TRT, FORCE>(p, A, flags, x0, y, z, inb, acc, has_link);
+  if (p.compute_force) block_force_reduce(acc, has_link, p.force + block_stripe());
+}
+
+// Pair kernel for any even row length and any faces: the pairs of a z plane are numbered row
+// after row (consecutive pairs are consecutive in memory whatever the row length, so no lane
+// idles at the row ends) and a thread finds its row with one multiplication (row_mul, row_shift).
+// Registers bound it: 38 populations live per thread.  Blocks of 128 threads, six per SM (80
+// registers) for BGK and five (96) for TRT, whose collision holds more; blocks of 256, three
+// per SM, spilled for TRT and ended less evenly (B200, us per step, FP32: channel 384x192x192
+// BGK 388 / 374, channel 210x187x171 TRT 218 / 211, periodic 250x190x190 TRT 288 / 256; FP16
+// deviations: channel 384x192x192 BGK 328 / 314).
+constexpr int ROWS_BLOCK = 128;
+template <class SP, bool ODD, bool TRT, int FORCE, bool FACES>
+__global__ void __launch_bounds__(ROWS_BLOCK, TRT ? 5 : 6) aa_rows_kernel(const __grid_constant__ AAParams p,
+                                                                                typename SP::S* __restrict__ A,
+                                                                                const uint8_t* __restrict__ flags) {
+  const Grid& g = p.g;
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, half = (unsigned)g.nx / 2;
+  const int z = blockIdx.y;
+  clear_record(p.zero_next);
+  if (ghost_plane(p, z)) return;  // whole block in a ghost plane
+  const unsigned row = __umulhi(t, p.row_mul) >> p.row_shift;
+  const bool inb = row < (unsigned)g.ny;
+  double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  bool has_link = false;
+  pair_cells<SP, ODD, TRT, FORCE, FACES>(p, A, flags, inb ? 2 * (int)(t - row * half) : 0, inb ? (int)row : 0, z, inb,
+                                         acc, has_link);
   if (p.compute_force) block_force_reduce(acc, has_link, p.force + block_stripe());
 }
 
@@ -1216,7 +1296,7 @@ __device__ __forceinline__ void pair_split_cells(const AAParams& p, typename SP:
 }
 
 template <class SP, bool TRT, int FORCE>
-__global__ void __launch_bounds__(256, (SP::MIN_BLOCKS > 2 ? 3 : 1)) aa_pair_split_kernel(const __grid_constant__ AAParams p,
+__global__ void __launch_bounds__(PAIR_X * SPLIT_ROWS, 6) aa_pair_split_kernel(const __grid_constant__ AAParams p,
                                                                                 typename SP::S* __restrict__ A,
                                                                                 const uint8_t* __restrict__ flags) {
   const Grid& g = p.g;
@@ -1240,7 +1320,7 @@ __global__ void __launch_bounds__(256, (SP::MIN_BLOCKS > 2 ? 3 : 1)) aa_pair_spl
 // four cells.  The cells collide in pairs, from the low and the high half2 of each word,
 // and pack back to half2 at once, which bounds the live registers.
 template <bool TRT, int FORCE>
-__global__ void __launch_bounds__(256, 2) aa_quad_even_kernel(const __grid_constant__ AAParams p,
+__global__ void __launch_bounds__(32 * QUAD_ROWS, 8) aa_quad_even_kernel(const __grid_constant__ AAParams p,
                                                               __half* __restrict__ A,
                                                               const uint8_t* __restrict__ flags) {
   using SP = StF16;
@@ -1358,7 +1438,7 @@ __device__ __forceinline__ void u4set(uint4& v, const int k, const uint32_t u) {
 }
 
 template <bool TRT, int FORCE>
-__global__ void __launch_bounds__(128, 3) aa_octo_even_kernel(const __grid_constant__ AAParams p,
+__global__ void __launch_bounds__(32 * OCTO_ROWS, 6) aa_octo_even_kernel(const __grid_constant__ AAParams p,
                                                               __half* __restrict__ A,
                                                               const uint8_t* __restrict__ flags) {
   using SP = StF16;
@@ -2069,9 +2149,18 @@ __global__ void aa_init_kernel(const InitParams p, typename SP::S* __restrict__ 
 template <class SP, bool ODD, bool TRT, int FORCE, bool FACES>
 static cudaError_t launch_one(const AAParams& p, void* A, const uint8_t* flags, dim3 grid, dim3 block,
                               cudaStream_t s) {
+  if constexpr (sizeof(typename SP::S) != 8) {
+    if (p.pair == 2) {
+      const dim3 rg((unsigned)(((long long)p.g.nx / 2 * p.g.ny + ROWS_BLOCK - 1) / ROWS_BLOCK), (unsigned)p.g.nz);
+      aa_rows_kernel<SP, ODD, TRT, FORCE, FACES><<<rg, ROWS_BLOCK, 0, s>>>(p, (typename SP::S*)A, flags);
+      return cudaGetLastError();
+    }
+  }
   if constexpr (!FACES) {
-    if (p.pair) {  // 64 x 4 threads, two cells each
-      const dim3 pb(64, 4, 1), pg((unsigned)(p.g.nx / 128), (unsigned)((p.g.ny + 3) / 4), (unsigned)p.g.nz);
+    if (p.pair) {
+      const unsigned px = (unsigned)(p.g.nx / 128), nz = (unsigned)p.g.nz;  // 64 threads along x, two cells each
+      const auto rows = [&](int n) { return (unsigned)((p.g.ny + n - 1) / n); };
+      const dim3 pb(PAIR_X, 1, 1), pg(px, (unsigned)p.g.ny, nz);
       if constexpr (ODD && SP::DEV) {
         if (p.quad) {  // whole rows: nx / 4 threads each, 128 threads (nx at most 512) or one row
           const int rows = p.g.nx <= 512 ? 512 / p.g.nx : 1;
@@ -2079,21 +2168,21 @@ static cudaError_t launch_one(const AAParams& p, void* A, const uint8_t* flags, 
               qg(1u, (unsigned)((p.g.ny + rows - 1) / rows), (unsigned)p.g.nz);
           aa_quad_odd_kernel<TRT, FORCE><<<qg, qb, 0, s>>>(p, (__half*)A, flags);
         } else {
-          aa_pair_split_kernel<SP, TRT, FORCE><<<pg, pb, 0, s>>>(p, (typename SP::S*)A, flags);
+          aa_pair_split_kernel<SP, TRT, FORCE><<<dim3(px, rows(SPLIT_ROWS), nz), dim3(PAIR_X, SPLIT_ROWS, 1), 0, s>>>(p, (typename SP::S*)A, flags);
         }
       } else if constexpr (!ODD && SP::DEV) {
-        if (p.quad == 2) {  // 32 x 4 threads, eight cells each (nx a multiple of 256)
-          const dim3 ob(32, 4, 1), og((unsigned)(p.g.nx / 256), (unsigned)((p.g.ny + 3) / 4), (unsigned)p.g.nz);
+        if (p.quad == 2) {  // 32 threads along x, eight cells each (nx a multiple of 256)
+          const dim3 ob(32, OCTO_ROWS, 1), og(px / 2, rows(OCTO_ROWS), nz);
           aa_octo_even_kernel<TRT, FORCE><<<og, ob, 0, s>>>(p, (__half*)A, flags);
-        } else if (p.quad) {  // 32 x 8 threads, four cells each
-          const dim3 qb(32, 8, 1), qg((unsigned)(p.g.nx / 128), (unsigned)((p.g.ny + 7) / 8), (unsigned)p.g.nz);
+        } else if (p.quad) {  // 32 threads along x, four cells each
+          const dim3 qb(32, QUAD_ROWS, 1), qg(px, rows(QUAD_ROWS), nz);
           aa_quad_even_kernel<TRT, FORCE><<<qg, qb, 0, s>>>(p, (__half*)A, flags);
         } else {
           aa_pair_kernel<SP, ODD, TRT, FORCE><<<pg, pb, 0, s>>>(p, (typename SP::S*)A, flags);
         }
       } else if constexpr (ODD && sizeof(typename SP::S) == 4) {
         if (p.xshuffle)
-          aa_pair_odd_kernel<SP, TRT, FORCE><<<pg, pb, 0, s>>>(p, (typename SP::S*)A, flags);
+          aa_pair_odd_kernel<SP, TRT, FORCE><<<dim3(px, rows(4), nz), dim3(64, 4, 1), 0, s>>>(p, (typename SP::S*)A, flags);
         else
           aa_pair_kernel<SP, ODD, TRT, FORCE><<<pg, pb, 0, s>>>(p, (typename SP::S*)A, flags);
       } else {

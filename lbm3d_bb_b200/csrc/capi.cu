@@ -76,6 +76,7 @@ struct lbm_ctx {
   // launch shape
   int bx = 0, by = 0;
   bool pair = false;  // FP16 pair kernel (see aa_pair_kernel)
+  bool rows = false;  // two cells per thread, any even row length and any faces (aa_rows_kernel)
   bool quad = false;  // FP16-deviation on the four-cell kernels
   bool xshuffle = false;  // FP32 odd phase on aa_pair_odd_kernel
   bool octo = false;  // FP16-deviation even phase on aa_octo_even_kernel
@@ -104,9 +105,19 @@ namespace {
 
 void default_block(lbm_ctx* c) {
   // rows of the box across threadIdx.x; whole warps, at most 256 threads (the step
-  // kernels' launch bound).  Rows that fit no such shape are padded to 32 lanes.
+  // kernels' launch bound).  Rows that fit no such shape are padded to 32 lanes.  Rows longer
+  // than 128 take blocks of 128 threads, 32, 64 or 128 wide.  32 x 4 is the fastest wherever
+  // faces or the reference step leave work to single lanes (B200, us per step against 128 x 1:
+  // FP32 channel 160x96x96 48.6 / 58.5, 384-wide equal, FP64 331x120x119 266 / 278, reference
+  // 480x240x4 26.6 / 28.7); fully periodic boxes take the widest of the three that pads least
+  // (FP32 192x96x96 62.4 / 68.7, FP64 383x120x120 128 x 1 318.7, 32 x 4 322.1).
   const int nx = c->g.nx;
   int bx = nx <= 128 ? nx : 128;
+  if (nx > 128) {
+    const bool periodic = !c->ref && c->g.per[0] && c->g.per[1] && c->g.per[2];
+    for (int w : {64, 32})
+      if (!periodic || (nx + w - 1) / w * w < (nx + bx - 1) / bx * bx) bx = w;
+  }
   int by = std::max(1, 128 / bx);
   while ((bx * by) % 32 != 0 && bx * (by + 1) <= 256) by++;
   if ((bx * by) % 32 != 0) {
@@ -414,6 +425,13 @@ void fill_aa_params(const lbm_ctx* c, AAParams& p, bool odd) {
     for (int a = 0; a < 3; a++) p.kin.center[a] = c->torque_center[a];
   p.compute_force = c->cfg.compute_force ? 1 : 0;
   p.links = c->links;
+  if (c->g.nx >= 4) {  // divisor d = nx / 2, 2^(l-1) < d <= 2^l: ceil(2^(31+l) / d) is exact below 2^31
+    const unsigned long long d = (unsigned long long)c->g.nx / 2;
+    int l = 1;
+    while ((1ull << l) < d) l++;
+    p.row_mul = (unsigned)(((1ull << (31 + l)) + d - 1) / d);
+    p.row_shift = (unsigned)(l - 1);
+  }
   const long long nx = c->g.nx, nxy = (long long)c->g.nx * c->g.ny, pl = c->g.plane;
   for (int d = 0; d < 19; d++) {
     const long long nb = cx(d) + nx * cy(d) + nxy * cz(d);
@@ -755,14 +773,24 @@ int32_t lbm_create(const lbm_config* cfg, int32_t device, lbm_ctx** out) {
                       (c->g.per[2] || halo_only(c));
     const bool wanted = env ? env[0] == '1' : cfg->storage != LBM_STORE_FP64;
     c->pair = fits && wanted;
+    // the same update for any even row length and any faces (aa_rows_kernel), from 1.4 M cells:
+    // smaller boxes do not fill the GPU with half the threads (B200, us per step, one cell /
+    // rows, FP32: channel 96x48x48 11.3 / 11.7, 128x96x96 39 / 40, 160x96x96 49.0 / 49.0,
+    // 192x120x120 86 / 82, 384x192x192 411 / 374; FP16 deviations 160x96x96 43.1 / 41.8).
+    // LBM3D_PAIR=1 / 0 forces it on / off
+    c->rows = !c->ref && !c->tma && !c->pair && cfg->nx % 2 == 0 && cfg->nx >= 4 && cfg->storage != LBM_STORE_FP64 &&
+              (env ? env[0] == '1' : c->g.N >= 1400000);
     // four cells per thread in the FP16-deviation even phase (aa_quad_even_kernel);
     // LBM3D_QUAD=0 keeps the pair kernels
     const char* q = std::getenv("LBM3D_QUAD");
     c->quad = c->pair && cfg->storage == LBM_STORE_FP16DEV && !(q && q[0] == '0');
     // eight cells per thread in the FP16-deviation even phase (16-byte words; nx a multiple
-    // of 256; 6 % faster than four cells on the 512^3 box on B200); LBM3D_OCTO=0 keeps four
+    // of 256): BGK boxes of 64 M cells and more, where it equals the four-cell kernel (512^3
+    // 2222 / 2210 us per step on B200); smaller ones run short of blocks (256x160x140 114 / 106)
+    // and TRT spills (256x160x140 with forces 201 / 153).  LBM3D_OCTO=1 / 0 forces it on / off
     const char* oc = std::getenv("LBM3D_OCTO");
-    c->octo = c->quad && cfg->nx % 256 == 0 && !(oc && oc[0] == '0');
+    c->octo = c->quad && cfg->nx % 256 == 0 &&
+              (oc ? oc[0] != '0' : cfg->collision == LBM_COLL_BGK && c->g.N >= (64LL << 20));
     // FP32 odd phase with the x-shifted directions moved as shuffled two-element words:
     // LBM3D_XSHUFFLE=1 (5 % slower than the pair kernel on the 512^3 box on B200)
     const char* xs = std::getenv("LBM3D_XSHUFFLE");
@@ -1038,7 +1066,7 @@ int32_t lbm_step(lbm_ctx* c, int32_t nsteps) {
       fill_aa_params(c, p, c->swapped);
       p.force = slot;
       p.zero_next = next;
-      p.pair = c->pair ? 1 : 0;
+      p.pair = c->pair ? 1 : (c->rows ? 2 : 0);
       p.quad = c->pair && c->quad ? (c->swapped ? (c->quad_odd ? 1 : 0) : (c->octo ? 2 : 1)) : 0;
       p.xshuffle = c->pair && c->xshuffle ? 1 : 0;
       if (c->tma) {

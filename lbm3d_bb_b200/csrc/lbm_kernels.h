@@ -40,7 +40,8 @@ struct AAParams {
   // per-node link words of NEAR nodes (see near_kernel): static no-slip links stay
   // on the fast path, everything else takes the general path
   const unsigned long long* links;
-  int pair;  // all axes periodic, nx % 128 == 0: two cells per thread (aa_pair_kernel)
+  int pair;  // two cells per thread: 1 all axes periodic, nx % 128 == 0 (aa_pair_kernel), 2 any even nx (aa_rows_kernel)
+  unsigned row_mul, row_shift;  // t / (nx / 2) = umulhi(t, row_mul) >> row_shift for t < 2^31 (pair == 2, nx >= 4)
   int quad;  // with pair, FP16-deviation: 1 four cells per thread (aa_quad_even/odd_kernel), 2 eight in the even phase (aa_octo_even_kernel)
   int xshuffle;  // with pair, FP32 odd phase: x-shifted directions as shuffled words (aa_pair_odd_kernel)
 };
