@@ -353,12 +353,27 @@ RefParams ref_params(const lbm_ctx* c, const Kinematics& kin, uint8_t solid_bit)
   return p;
 }
 
+// t / (nx / 2) = umulhi(t, mul) >> shift for t < 2^31, nx >= 4: with 2^(l-1) < d <= 2^l,
+// ceil(2^(31+l) / d) is exact below 2^31.
+void row_divisor(int nx, unsigned& mul, unsigned& shift) {
+  if (nx < 4) return;
+  const unsigned long long d = (unsigned long long)nx / 2;
+  int l = 1;
+  while ((1ull << l) < d) l++;
+  mul = (unsigned)(((1ull << (31 + l)) + d - 1) / d);
+  shift = (unsigned)(l - 1);
+}
+
 ReadParams read_params(const lbm_ctx* c) {
   ReadParams p{};
   p.g = c->g;
+  for (int d = 0; d < 19; d++)
+    p.off[d] = opp(d) * c->g.plane - (cx(d) + (long long)c->g.nx * cy(d) + (long long)c->g.nx * c->g.ny * cz(d));
+  row_divisor(c->g.nx, p.row_mul, p.row_shift);
   p.rho0 = c->cfg.rho0;
   p.swapped = c->swapped ? 1 : 0;
   p.solid_bit = F_SOLID_PREV;
+  p.links = c->links;
   for (int a = 0; a < 3; a++) p.gacc[a] = c->cfg.accel[a];
   return p;
 }
@@ -425,13 +440,7 @@ void fill_aa_params(const lbm_ctx* c, AAParams& p, bool odd) {
     for (int a = 0; a < 3; a++) p.kin.center[a] = c->torque_center[a];
   p.compute_force = c->cfg.compute_force ? 1 : 0;
   p.links = c->links;
-  if (c->g.nx >= 4) {  // divisor d = nx / 2, 2^(l-1) < d <= 2^l: ceil(2^(31+l) / d) is exact below 2^31
-    const unsigned long long d = (unsigned long long)c->g.nx / 2;
-    int l = 1;
-    while ((1ull << l) < d) l++;
-    p.row_mul = (unsigned)(((1ull << (31 + l)) + d - 1) / d);
-    p.row_shift = (unsigned)(l - 1);
-  }
+  row_divisor(c->g.nx, p.row_mul, p.row_shift);
   const long long nx = c->g.nx, nxy = (long long)c->g.nx * c->g.ny, pl = c->g.plane;
   for (int d = 0; d < 19; d++) {
     const long long nb = cx(d) + nx * cy(d) + nxy * cz(d);
@@ -1122,6 +1131,7 @@ int32_t lbm_get_force_history(lbm_ctx* c, int64_t first, int32_t count, double* 
                                 (size_t)n * FORCE_RECORD * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
                 "D2H force"))
       return LBM_ERR_CUDA;
+    k += n;
   }
   if (c->cuda(cudaStreamSynchronize(c->stream), "force")) return LBM_ERR_CUDA;
   for (int32_t k = 0; k < count; k++)

@@ -101,8 +101,11 @@ struct ReadParams {
   Grid g;
   double rho0;
   int swapped;        // AA: state in swapped layout (after an even phase)
-  uint8_t solid_bit;  // flag bit holding the solids of the last completed step
+  uint8_t solid_bit;  // flag bit holding the solids of the last completed step (F_SOLID_PREV)
   double gacc[3];
+  const unsigned long long* links;  // link words (near_kernel): bits 18..35 name the neighbours with solid_bit
+  long long off[19];                // swapped layout: element offset of direction d's slot from an interior node
+  unsigned row_mul, row_shift;      // as in AAParams
 };
 
 struct ExportOut {
@@ -140,7 +143,30 @@ __device__ __forceinline__ double import_value(const InitParams& p, const Grid& 
   return p.f_dtype == LBM_DTYPE_F64 ? ((const double*)p.f_in)[k] : (double)((const float*)p.f_in)[k];
 }
 
-// Writes one node's populations and/or moments (config-mode moments: u = j/rho + g/2).
+// Exported moments of one node (config mode: u = j/rho + g/2, zero in a solid).
+template <class C>
+__device__ __forceinline__ void export_moments(const C* f, bool solid, const double* gacc, C& r, C& ux, C& uy, C& uz) {
+  C jx = C(0), jy = C(0), jz = C(0);
+  r = f[0];
+#pragma unroll
+  for (int d = 1; d < 19; d++) r += f[d];
+#pragma unroll
+  for (int d = 0; d < 19; d++) {
+    jx += f[d] * C(cx(d));
+    jy += f[d] * C(cy(d));
+    jz += f[d] * C(cz(d));
+  }
+  ux = uy = uz = C(0);
+  if (!solid) {
+    ux = jx / r + C(0.5) * C(gacc[0]);
+    uy = jy / r + C(0.5) * C(gacc[1]);
+    uz = jz / r + C(0.5) * C(gacc[2]);
+  } else {
+    r = C(0);
+  }
+}
+
+// Writes one node's populations and/or moments.
 template <class C>
 __device__ __forceinline__ void export_node(const ExportOut& o, const Grid& g, long long i, const C* f,
                                             bool solid, const double* gacc) {
@@ -152,23 +178,8 @@ __device__ __forceinline__ void export_node(const ExportOut& o, const Grid& g, l
     }
   }
   if (o.rho || o.u || o.v || o.w) {
-    C r = f[0], jx = C(0), jy = C(0), jz = C(0);
-#pragma unroll
-    for (int d = 1; d < 19; d++) r += f[d];
-#pragma unroll
-    for (int d = 0; d < 19; d++) {
-      jx += f[d] * C(cx(d));
-      jy += f[d] * C(cy(d));
-      jz += f[d] * C(cz(d));
-    }
-    C ux = C(0), uy = C(0), uz = C(0);
-    if (!solid) {
-      ux = jx / r + C(0.5) * C(gacc[0]);
-      uy = jy / r + C(0.5) * C(gacc[1]);
-      uz = jz / r + C(0.5) * C(gacc[2]);
-    } else {
-      r = C(0);
-    }
+    C r, ux, uy, uz;
+    export_moments<C>(f, solid, gacc, r, ux, uy, uz);
     if (o.rho) put<C>(o.rho, i, o.m_dtype, r);
     if (o.u) put<C>(o.u, i, o.m_dtype, ux);
     if (o.v) put<C>(o.v, i, o.m_dtype, uy);
