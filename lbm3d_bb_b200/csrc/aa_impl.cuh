@@ -771,6 +771,7 @@ __global__ void __launch_bounds__(256, SP::MIN_BLOCKS) aa_step_kernel(const __gr
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int z = blockIdx.z;
   const bool inb = (x < g.nx) && (y < g.ny);
+  chain_begin();
   clear_record(p.zero_next);  // the next step's force record (read by the next launch only)
   if (ghost_plane(p, z)) return;  // whole block in a ghost plane
   double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -1031,6 +1032,7 @@ __global__ void __launch_bounds__(PAIR_X, pair_blocks<SP, TRT>()) aa_pair_kernel
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int z = blockIdx.z;
   const bool inb = x0 < g.nx && y < g.ny;
+  chain_begin();
   clear_record(p.zero_next);
   if (ghost_plane(p, z)) return;  // whole block in a ghost plane
   double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -1055,6 +1057,7 @@ __global__ void __launch_bounds__(ROWS_BLOCK, TRT ? 5 : 6) aa_rows_kernel(const 
   const Grid& g = p.g;
   const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, half = (unsigned)g.nx / 2;
   const int z = blockIdx.y;
+  chain_begin();
   clear_record(p.zero_next);
   if (ghost_plane(p, z)) return;  // whole block in a ghost plane
   const unsigned row = __umulhi(t, p.row_mul) >> p.row_shift;
@@ -1087,6 +1090,7 @@ __global__ void __launch_bounds__(256, (SP::MIN_BLOCKS > 2 ? 3 : 1)) aa_pair_odd
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int z = blockIdx.z;
   const bool inb = x0 < g.nx && y < g.ny;
+  chain_begin();
   clear_record(p.zero_next);
   if (ghost_plane(p, z)) return;  // whole block in a ghost plane
   double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -1306,6 +1310,7 @@ __global__ void __launch_bounds__(PAIR_X * SPLIT_ROWS, 6) aa_pair_split_kernel(c
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int z = blockIdx.z;
   const bool inb = x0 < g.nx && y < g.ny;
+  chain_begin();
   clear_record(p.zero_next);
   if (ghost_plane(p, z)) return;  // whole block in a ghost plane
   double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -1332,6 +1337,7 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 8) aa_quad_even_kernel(const _
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int z = blockIdx.z;
   const bool inb = x0 < g.nx && y < g.ny;
+  chain_begin();
   clear_record(p.zero_next);
   if (ghost_plane(p, z)) return;  // whole block in a ghost plane
   double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -1450,6 +1456,7 @@ __global__ void __launch_bounds__(32 * OCTO_ROWS, 6) aa_octo_even_kernel(const _
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int z = blockIdx.z;
   const bool inb = x0 < g.nx && y < g.ny;
+  chain_begin();
   clear_record(p.zero_next);
   if (ghost_plane(p, z)) return;  // whole block in a ghost plane
   double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -1601,6 +1608,7 @@ __global__ void __launch_bounds__(256, 2) aa_quad_odd_kernel(const __grid_consta
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int z = blockIdx.z;
   const bool inb = y < g.ny;
+  chain_begin();
   clear_record(p.zero_next);
   if (ghost_plane(p, z)) return;  // whole block in a ghost plane
   // exchange: the element of each x-shifted direction (slot xslot(d)) that enters the
@@ -2262,8 +2270,7 @@ static cudaError_t launch_one(const AAParams& p, void* A, const uint8_t* flags, 
   if constexpr (sizeof(typename SP::S) != 8) {
     if (p.pair == 2) {
       const dim3 rg((unsigned)(((long long)p.g.nx / 2 * p.g.ny + ROWS_BLOCK - 1) / ROWS_BLOCK), (unsigned)p.g.nz);
-      aa_rows_kernel<SP, ODD, TRT, FORCE, FACES><<<rg, ROWS_BLOCK, 0, s>>>(p, (typename SP::S*)A, flags);
-      return cudaGetLastError();
+      return launch_chained(aa_rows_kernel<SP, ODD, TRT, FORCE, FACES>, rg, ROWS_BLOCK, s, p, (typename SP::S*)A, flags);
     }
   }
   if constexpr (!FACES) {
@@ -2276,29 +2283,28 @@ static cudaError_t launch_one(const AAParams& p, void* A, const uint8_t* flags, 
           const int rows = p.g.nx <= 512 ? 512 / p.g.nx : 1;
           const dim3 qb((unsigned)(p.g.nx / 4), (unsigned)rows, 1),
               qg(1u, (unsigned)((p.g.ny + rows - 1) / rows), (unsigned)p.g.nz);
-          aa_quad_odd_kernel<TRT, FORCE><<<qg, qb, 0, s>>>(p, (__half*)A, flags);
+          return launch_chained(aa_quad_odd_kernel<TRT, FORCE>, qg, qb, s, p, (__half*)A, flags);
         } else {
-          aa_pair_split_kernel<SP, TRT, FORCE><<<dim3(px, rows(SPLIT_ROWS), nz), dim3(PAIR_X, SPLIT_ROWS, 1), 0, s>>>(p, (typename SP::S*)A, flags);
+          return launch_chained(aa_pair_split_kernel<SP, TRT, FORCE>, dim3(px, rows(SPLIT_ROWS), nz), dim3(PAIR_X, SPLIT_ROWS, 1), s, p, (typename SP::S*)A, flags);
         }
       } else if constexpr (!ODD && SP::DEV) {
         if (p.quad == 2) {  // 32 threads along x, eight cells each (nx a multiple of 256)
           const dim3 ob(32, OCTO_ROWS, 1), og(px / 2, rows(OCTO_ROWS), nz);
-          aa_octo_even_kernel<TRT, FORCE><<<og, ob, 0, s>>>(p, (__half*)A, flags);
+          return launch_chained(aa_octo_even_kernel<TRT, FORCE>, og, ob, s, p, (__half*)A, flags);
         } else if (p.quad) {  // 32 threads along x, four cells each
           const dim3 qb(32, QUAD_ROWS, 1), qg(px, rows(QUAD_ROWS), nz);
-          aa_quad_even_kernel<TRT, FORCE><<<qg, qb, 0, s>>>(p, (__half*)A, flags);
+          return launch_chained(aa_quad_even_kernel<TRT, FORCE>, qg, qb, s, p, (__half*)A, flags);
         } else {
-          aa_pair_kernel<SP, ODD, TRT, FORCE><<<pg, pb, 0, s>>>(p, (typename SP::S*)A, flags);
+          return launch_chained(aa_pair_kernel<SP, ODD, TRT, FORCE>, pg, pb, s, p, (typename SP::S*)A, flags);
         }
       } else if constexpr (ODD && sizeof(typename SP::S) == 4) {
         if (p.xshuffle)
-          aa_pair_odd_kernel<SP, TRT, FORCE><<<dim3(px, rows(4), nz), dim3(64, 4, 1), 0, s>>>(p, (typename SP::S*)A, flags);
+          return launch_chained(aa_pair_odd_kernel<SP, TRT, FORCE>, dim3(px, rows(4), nz), dim3(64, 4, 1), s, p, (typename SP::S*)A, flags);
         else
-          aa_pair_kernel<SP, ODD, TRT, FORCE><<<pg, pb, 0, s>>>(p, (typename SP::S*)A, flags);
+          return launch_chained(aa_pair_kernel<SP, ODD, TRT, FORCE>, pg, pb, s, p, (typename SP::S*)A, flags);
       } else {
-        aa_pair_kernel<SP, ODD, TRT, FORCE><<<pg, pb, 0, s>>>(p, (typename SP::S*)A, flags);
+        return launch_chained(aa_pair_kernel<SP, ODD, TRT, FORCE>, pg, pb, s, p, (typename SP::S*)A, flags);
       }
-      return cudaGetLastError();
     }
   }
   if (p.tma.enabled) {
@@ -2321,8 +2327,7 @@ static cudaError_t launch_one(const AAParams& p, void* A, const uint8_t* flags, 
     kern<<<(unsigned)nb, p.tma.tw, smem, s>>>(p, (typename SP::S*)A, flags);
     return cudaGetLastError();
   }
-  aa_step_kernel<SP, ODD, TRT, FORCE, FACES><<<grid, block, 0, s>>>(p, (typename SP::S*)A, flags);
-  return cudaGetLastError();
+  return launch_chained(aa_step_kernel<SP, ODD, TRT, FORCE, FACES>, grid, block, s, p, (typename SP::S*)A, flags);
 }
 
 template <class SP>

@@ -138,11 +138,11 @@ __global__ void spheres_kernel(const Grid g, const double* __restrict__ xyzr, in
 // from the pose of the last completed step; NEAR is recomputed afterwards.
 __global__ void moving_kernel(const __grid_constant__ FlagParams p, uint8_t* flags) {
   const Grid& g = p.g;
-  const int bx = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ex = p.box.hi[0] - p.box.lo[0] + 1;
-  if (bx >= ex) return;
+  chain_begin();
+  const int bx = blockIdx.x * blockDim.x + threadIdx.x, by = blockIdx.y * blockDim.y + threadIdx.y;
+  if (bx > p.box.hi[0] - p.box.lo[0] || by > p.box.hi[1] - p.box.lo[1]) return;
   const int x = wrapc(p.box.lo[0] + bx, g.nx);
-  const int y = wrapc(p.box.lo[1] + (int)blockIdx.y, g.ny);
+  const int y = wrapc(p.box.lo[1] + by, g.ny);
   const int z = wrapc(p.box.lo[2] + (int)blockIdx.z, g.nz);
   const long long i = node_index(g, x, y, z);
   const uint8_t st = flags[i] & F_STATIC;
@@ -162,11 +162,11 @@ __global__ void moving_kernel(const __grid_constant__ FlagParams p, uint8_t* fla
 // it belongs to the moving body now (sources outside a non-periodic face: no bit).
 __global__ void near_kernel(const Grid g, int mode, const Box box, uint8_t* flags,
                             unsigned long long* links) {
-  const int bx = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ex = box.hi[0] - box.lo[0] + 1;
-  if (bx >= ex) return;
+  chain_begin();
+  const int bx = blockIdx.x * blockDim.x + threadIdx.x, by = blockIdx.y * blockDim.y + threadIdx.y;
+  if (bx > box.hi[0] - box.lo[0] || by > box.hi[1] - box.lo[1]) return;
   const int x = wrapc(box.lo[0] + bx, g.nx);
-  const int y = wrapc(box.lo[1] + (int)blockIdx.y, g.ny);
+  const int y = wrapc(box.lo[1] + by, g.ny);
   const int z = wrapc(box.lo[2] + (int)blockIdx.z, g.nz);
   const long long i = node_index(g, x, y, z);
   const uint8_t fl = flags[i];
@@ -359,9 +359,9 @@ __global__ void sync_prev_kernel(const Grid g, uint8_t* flags) {
 }
 
 // ---- launchers --------------------------------------------------------------------------------------
-static dim3 box_grid(const Box& b, int bx) {
+static dim3 box_grid(const Box& b, int bx, int by = 1) {
   const int ex = b.hi[0] - b.lo[0] + 1, ey = b.hi[1] - b.lo[1] + 1, ez = b.hi[2] - b.lo[2] + 1;
-  return dim3((unsigned)((ex + bx - 1) / bx), (unsigned)ey, (unsigned)ez);
+  return dim3((unsigned)((ex + bx - 1) / bx), (unsigned)((ey + by - 1) / by), (unsigned)ez);
 }
 
 cudaError_t geo_launch_static(const Grid& g, const BodyDev& b, const Box& box, uint8_t* flags, cudaStream_t s) {
@@ -376,14 +376,13 @@ cudaError_t geo_launch_spheres(const Grid& g, const double* xyzr, int count, uin
 }
 
 cudaError_t geo_launch_moving(const FlagParams& p, uint8_t* flags, cudaStream_t s) {
-  moving_kernel<<<box_grid(p.box, 128), 128, 0, s>>>(p, flags);
-  return cudaGetLastError();
+  // a body's box is some thirty cells wide: one warp per row, four rows per block
+  return launch_chained(moving_kernel, box_grid(p.box, 32, 4), dim3(32, 4), s, p, flags);
 }
 
 cudaError_t geo_launch_near(const Grid& g, int mode, const Box& box, uint8_t* flags, unsigned long long* links,
                             cudaStream_t s) {
-  near_kernel<<<box_grid(box, 128), 128, 0, s>>>(g, mode, box, flags, links);
-  return cudaGetLastError();
+  return launch_chained(near_kernel, box_grid(box, 32, 4), dim3(32, 4), s, g, mode, box, flags, links);
 }
 
 cudaError_t geo_launch_sync_prev(const Grid& g, uint8_t* flags, cudaStream_t s) {

@@ -41,34 +41,22 @@ __host__ __device__ __forceinline__ T wgt(int d) {
 
 // ---- launchers (the lattice follows the grid: g.q = 19 or 27) ------------------------
 template <class T, bool TRT, int QN>
-static void step_one(const RefParams& p, const void* Fp, const void* Rp, void* Fn, void* Rn, const uint8_t* flags,
+static cudaError_t step_one(const RefParams& p, const void* Fp, const void* Rp, void* Fn, void* Rn, const uint8_t* flags,
                      dim3 grid, dim3 block, cudaStream_t s) {
   if constexpr (QN == 27)
-    ref27::ref_step_kernel<T, TRT><<<grid, block, 0, s>>>(p, (const T*)Fp, (const T*)Rp, (T*)Fn, (T*)Rn, flags);
+    return launch_chained(ref27::ref_step_kernel<T, TRT>, grid, block, s, p, (const T*)Fp, (const T*)Rp, (T*)Fn, (T*)Rn, flags);
   else
-    ref19::ref_step_kernel<T, TRT><<<grid, block, 0, s>>>(p, (const T*)Fp, (const T*)Rp, (T*)Fn, (T*)Rn, flags);
+    return launch_chained(ref19::ref_step_kernel<T, TRT>, grid, block, s, p, (const T*)Fp, (const T*)Rp, (T*)Fn, (T*)Rn, flags);
 }
 
 cudaError_t ref_launch_step(bool fp64, bool trt, const RefParams& p, const void* Fp, const void* Rp,
                             void* Fn, void* Rn, const uint8_t* flags, dim3 grid, dim3 block,
                             cudaStream_t s) {
-  const bool q27 = p.g.q == 27;
-  if (fp64) {
-    if (trt)
-      q27 ? step_one<double, true, 27>(p, Fp, Rp, Fn, Rn, flags, grid, block, s)
-          : step_one<double, true, 19>(p, Fp, Rp, Fn, Rn, flags, grid, block, s);
-    else
-      q27 ? step_one<double, false, 27>(p, Fp, Rp, Fn, Rn, flags, grid, block, s)
-          : step_one<double, false, 19>(p, Fp, Rp, Fn, Rn, flags, grid, block, s);
-  } else {
-    if (trt)
-      q27 ? step_one<float, true, 27>(p, Fp, Rp, Fn, Rn, flags, grid, block, s)
-          : step_one<float, true, 19>(p, Fp, Rp, Fn, Rn, flags, grid, block, s);
-    else
-      q27 ? step_one<float, false, 27>(p, Fp, Rp, Fn, Rn, flags, grid, block, s)
-          : step_one<float, false, 19>(p, Fp, Rp, Fn, Rn, flags, grid, block, s);
-  }
-  return cudaGetLastError();
+  const auto step = p.g.q == 27 ? (fp64 ? (trt ? step_one<double, true, 27> : step_one<double, false, 27>)
+                                        : (trt ? step_one<float, true, 27> : step_one<float, false, 27>))
+                                : (fp64 ? (trt ? step_one<double, true, 19> : step_one<double, false, 19>)
+                                        : (trt ? step_one<float, true, 19> : step_one<float, false, 19>));
+  return step(p, Fp, Rp, Fn, Rn, flags, grid, block, s);
 }
 
 template <class T>

@@ -251,6 +251,7 @@ __global__ void __launch_bounds__(256) ref_step_kernel(const __grid_constant__ R
   const int z = blockIdx.z;
   double acc[6] = {0, 0, 0, 0, 0, 0};
   bool has = false;
+  chain_begin();
   clear_record(p.zero_next);  // the next step's force record (read by the next launch only)
   if (x < g.nx && y < g.ny) {
     const long long i = node_index(g, x, y, z);
