@@ -256,7 +256,8 @@ int sync_flags(lbm_ctx* c) {
   r = box_union(r, body_box(c, b, c->pose_last_step.center, 2));
   r = box_union(r, body_box(c, b, c->pose_latest.center, 2));
   Box rn = dilate(r, 1);
-  if (box_clamp(c, r)) {
+  const bool flags_box = box_clamp(c, r), near_box = box_clamp(c, rn);
+  if (flags_box) {  // then rn, which holds r, is not empty
     FlagParams p{};
     p.g = c->g;
     p.mode = c->cfg.mode;
@@ -265,10 +266,9 @@ int sync_flags(lbm_ctx* c) {
     p.body_prev = to_dev(c, b, &c->pose_last_step);
     p.has_moving = 1;
     c->launches++;
-    int rc = c->cuda(geo_launch_moving(p, c->flags, c->stream), "moving-body flags");
+    int rc = c->cuda(geo_launch_body(p, rn, c->flags, c->links, c->stream), "moving-body flags");
     if (rc) return rc;
-  }
-  if (box_clamp(c, rn)) {
+  } else if (near_box) {
     c->launches++;
     int rc = c->cuda(geo_launch_near(c->g, c->cfg.mode, rn, c->flags, c->links, c->stream), "near flags");
     if (rc) return rc;
@@ -1075,7 +1075,13 @@ int32_t lbm_step(lbm_ctx* c, int32_t nsteps) {
       fill_aa_params(c, p, c->swapped);
       p.force = slot;
       p.zero_next = next;
-      p.pair = c->pair ? 1 : (c->rows ? 2 : 0);
+      // a moving body in a box with faces: one cell per thread, links on the fast path
+      // up to 6 M cells, 2 M for BGK in FP16 deviations (B200, us per step, other rule / this:
+      // FP32 TRT 192x96x96 87 / 79, BGK 240x150x140 182 / 174, 384x205x199 466 / 478; FP16
+      // TRT 192x96x96 75 / 67, BGK 240x150x140 159 / 163)
+      const bool bgk16 = c->cfg.storage == LBM_STORE_FP16DEV && !trt;
+      p.move = c->has_moving && has_faces(c) && c->g.N < (bgk16 ? 2000000 : 6000000);
+      p.pair = c->pair ? 1 : (c->rows && !p.move ? 2 : 0);
       p.quad = c->pair && c->quad ? (c->swapped ? (c->quad_odd ? 1 : 0) : (c->octo ? 2 : 1)) : 0;
       p.xshuffle = c->pair && c->xshuffle ? 1 : 0;
       if (c->tma) {

@@ -11,6 +11,8 @@
 // CPU restatement built with -ffp-contract=off, so flags and links are bit-exact.
 #include <mutex>
 
+#include <initializer_list>
+
 #include "lbm_internal.cuh"
 #include "lbm_kernels.h"
 #include "shapes.cuh"
@@ -358,6 +360,86 @@ __global__ void sync_prev_kernel(const Grid g, uint8_t* flags) {
   flags[i] = v;
 }
 
+// moving_kernel followed by near_kernel on the box `rn` (the moving body's box p.box, dilated by
+// one node) in one launch: a block evaluates the flags of its tile and of the nodes around it into
+// shared memory, where near_kernel's rule reads them.  A node inside p.box takes its bits from the
+// static bit, which never changes, and the two poses; any other node keeps what its byte says but
+// for NEAR, which only its own block writes.  So nothing a block reads depends on another's
+// writes.  Two dependent launches cost 21 us of an 80 us step of the 192x96x96 channel with a
+// moving sphere on B200 (latency: the box has 22,000 nodes), this one 17.
+constexpr int FT_X = 32, FT_Y = 4, FT_Z = 2;
+
+// c within one period of [0, n)
+__device__ __forceinline__ int wrap1(int c, int n) { return c < 0 ? c + n : (c >= n ? c - n : c); }
+
+__device__ __forceinline__ bool in_box(const Grid& g, const Box& b, int x, int y, int z) {
+  const int c[3] = {x, y, z}, n[3] = {g.nx, g.ny, g.nz};
+#pragma unroll
+  for (int a = 0; a < 3; a++)  // boxes start in [0, n) (geo_launch_body)
+    if (wrap1(c[a] - b.lo[a], n[a]) > b.hi[a] - b.lo[a]) return false;
+  return true;
+}
+
+__global__ void __launch_bounds__(FT_X* FT_Y* FT_Z) body_flags_kernel(const __grid_constant__ FlagParams p, const Box rn,
+                                                                      uint8_t* flags, unsigned long long* links) {
+  chain_begin();
+  const Grid& g = p.g;
+  constexpr int HX = FT_X + 2, HY = FT_Y + 2, HZ = FT_Z + 2;
+  __shared__ uint8_t tile[HZ][HY][HX];  // 0 outside the box of nodes
+  const int n3[3] = {g.nx, g.ny, g.nz};
+  const bool wrap = p.mode == LBM_MODE_CONFIG;
+  const int o[3] = {rn.lo[0] + (int)blockIdx.x * FT_X, rn.lo[1] + (int)blockIdx.y * FT_Y,
+                    rn.lo[2] + (int)blockIdx.z * FT_Z};
+  const int tid = threadIdx.x + FT_X * (threadIdx.y + FT_Y * threadIdx.z);
+  // a node beyond a non-periodic end (every end in reference mode) is no neighbour
+  const auto node = [&](int a, int c) -> int {
+    if (c >= 0 && c < n3[a]) return c;
+    return wrap && g.per[a] ? wrap1(c, n3[a]) : -1;
+  };
+  for (int k = tid; k < HX * HY * HZ; k += FT_X * FT_Y * FT_Z) {
+    const int hx = k % HX, hy = k / HX % HY, hz = k / (HX * HY);
+    const int c[3] = {o[0] + hx - 1, o[1] + hy - 1, o[2] + hz - 1};
+    uint8_t v = 0;
+    const int x = node(0, c[0]), y = node(1, c[1]), z = node(2, c[2]);
+    const bool used = c[0] <= rn.hi[0] + 1 && c[1] <= rn.hi[1] + 1 && c[2] <= rn.hi[2] + 1;
+    if (used && (x | y | z) >= 0) {
+      const uint8_t old = flags[node_index(g, x, y, z)];
+      if (in_box(g, p.box, x, y, z)) {
+        v = (old & F_STATIC) ? (uint8_t)(F_STATIC | F_SOLID | F_SOLID_PREV) : (uint8_t)0;
+        if (inside_body(p.body, g, x, y, z)) v |= F_MOVING | F_SOLID;
+        if (inside_body(p.body_prev, g, x, y, z)) v |= F_MOVING_PREV | F_SOLID_PREV;
+      } else {
+        v = old & (uint8_t)~F_NEAR;
+      }
+    }
+    tile[hz][hy][hx] = v;
+  }
+  __syncthreads();
+  const int ux = o[0] + (int)threadIdx.x, uy = o[1] + (int)threadIdx.y, uz = o[2] + (int)threadIdx.z;
+  if (ux > rn.hi[0] || uy > rn.hi[1] || uz > rn.hi[2]) return;
+  const int x = wrap1(ux, g.nx), y = wrap1(uy, g.ny), z = wrap1(uz, g.nz);
+  const long long i = node_index(g, x, y, z);
+  const int tx = threadIdx.x + 1, ty = threadIdx.y + 1, tz = threadIdx.z + 1;
+  const uint8_t fl = tile[tz][ty][tx];
+  const bool sc = fl & F_SOLID, sp = fl & F_SOLID_PREV;
+  bool near = sp && !sc;
+  unsigned long long lw = 0;
+#pragma unroll
+  for (int d = 0; d < 18; d++) {
+    const uint8_t fn = tile[tz - cz(d)][ty - cy(d)][tx - cx(d)];
+    if (fn & (F_SOLID | F_SOLID_PREV)) near = true;
+    if (fn & F_SOLID) lw |= 1ull << d;
+    if (fn & F_SOLID_PREV) lw |= 1ull << (18 + d);
+    if (fn & F_MOVING) lw |= 1ull << (36 + d);
+  }
+  if (g.q == 27)
+    for (int d = 18; d < 26; d++)
+      if (tile[tz - cz27(d)][ty - cy27(d)][tx - cx27(d)] & (F_SOLID | F_SOLID_PREV)) near = true;
+  near = near && (!sc || !sp);
+  flags[i] = near ? (uint8_t)(fl | F_NEAR) : fl;
+  if (links) links[i] = lw;
+}
+
 // ---- launchers --------------------------------------------------------------------------------------
 static dim3 box_grid(const Box& b, int bx, int by = 1) {
   const int ex = b.hi[0] - b.lo[0] + 1, ey = b.hi[1] - b.lo[1] + 1, ez = b.hi[2] - b.lo[2] + 1;
@@ -383,6 +465,25 @@ cudaError_t geo_launch_moving(const FlagParams& p, uint8_t* flags, cudaStream_t 
 cudaError_t geo_launch_near(const Grid& g, int mode, const Box& box, uint8_t* flags, unsigned long long* links,
                             cudaStream_t s) {
   return launch_chained(near_kernel, box_grid(box, 32, 4), dim3(32, 4), s, g, mode, box, flags, links);
+}
+
+cudaError_t geo_launch_body(const FlagParams& params, const Box& box, uint8_t* flags, unsigned long long* links,
+                            cudaStream_t s) {
+  // a body may be given any number of periods away: boxes that start in [0, n) (a box is shorter
+  // than the axis or all of it) let the kernel wrap with one addition
+  FlagParams p = params;
+  Box rn = box;
+  const int n3[3] = {p.g.nx, p.g.ny, p.g.nz};
+  for (Box* b : {&p.box, &rn})
+    for (int a = 0; a < 3; a++) {
+      int shift = b->lo[a] % n3[a];
+      shift = (shift < 0 ? shift + n3[a] : shift) - b->lo[a];
+      b->lo[a] += shift;
+      b->hi[a] += shift;
+    }
+  const dim3 grid((unsigned)((rn.hi[0] - rn.lo[0] + FT_X) / FT_X), (unsigned)((rn.hi[1] - rn.lo[1] + FT_Y) / FT_Y),
+                  (unsigned)((rn.hi[2] - rn.lo[2] + FT_Z) / FT_Z));
+  return launch_chained(body_flags_kernel, grid, dim3(FT_X, FT_Y, FT_Z), s, p, rn, flags, links);
 }
 
 cudaError_t geo_launch_sync_prev(const Grid& g, uint8_t* flags, cudaStream_t s) {

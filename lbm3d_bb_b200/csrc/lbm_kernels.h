@@ -41,6 +41,7 @@ struct AAParams {
   // on the fast path, everything else takes the general path
   const unsigned long long* links;
   int pair;  // two cells per thread: 1 all axes periodic, nx % 128 == 0 (aa_pair_kernel), 2 any even nx (aa_rows_kernel)
+  int move;  // one cell per thread, links to the moving body on the fast path (boxes with faces)
   unsigned row_mul, row_shift;  // t / (nx / 2) = umulhi(t, row_mul) >> row_shift for t < 2^31 (pair == 2, nx >= 4)
   int quad;  // with pair, FP16-deviation: 1 four cells per thread (aa_quad_even/odd_kernel), 2 eight in the even phase (aa_octo_even_kernel)
   int xshuffle;  // with pair, FP32 odd phase: x-shifted directions as shuffled words (aa_pair_odd_kernel)
@@ -314,6 +315,8 @@ cudaError_t geo_launch_spheres(const Grid& g, const double* xyzr, int count, uin
 cudaError_t geo_launch_moving(const FlagParams& p, uint8_t* flags, cudaStream_t s);
 cudaError_t geo_launch_near(const Grid& g, int mode, const Box& box, uint8_t* flags, unsigned long long* links,
                             cudaStream_t s);
+// Both for a moving body, in one launch: flags in p.box, NEAR bits and link words in rn.
+cudaError_t geo_launch_body(const FlagParams& p, const Box& rn, uint8_t* flags, unsigned long long* links, cudaStream_t s);
 cudaError_t geo_launch_sync_prev(const Grid& g, uint8_t* flags, cudaStream_t s);
 // Link export: counts per node (cur solid bits), exclusive scan, CSR fill.
 cudaError_t geo_links(const Grid& g, int mode, const uint8_t* flags, uint8_t solid_bit, int32_t* d_count,

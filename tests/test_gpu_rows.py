@@ -118,3 +118,34 @@ def test_odd_rows_take_the_one_cell_kernel(gpu, oracle_lib):
     finally:
         g.close()
         o.close()
+
+
+@pytest.mark.parametrize("shape,center", [((24, 16, 18), (0.7, 8.1, 17.2)), ((17, 40, 19), (45.0, 39.0, -30.4)),
+                                          ((70, 9, 10), (35.2, 4.4, 5.1))])
+def test_body_flags_across_wraps(gpu, oracle_lib, shape, center):
+    """A moving sphere's flags and links, bit for bit: boxes that wrap, that start periods away
+    from the origin, that are as long as the axis, that need several tiles."""
+    from lbm3d_bb_b200 import abi
+
+    runs = []
+    for cls, kw in ((Domain, dict(storage="fp32")), (OracleDomain, dict(precision="fp64"))):
+        d = cls(*shape, collision="BGK", faces=("periodic",) * 6, omega_p=1.2, **kw)
+        d.add_spheres(np.array([[shape[0] / 2, 3.0, 4.0, 2.2]]))
+        d.add_body(abi.make_body(abi.BODY_SPHERE, center, radius=4.3, moving=True))
+        d.init_equilibrium()
+        runs.append(d)
+    try:
+        for n in range(6):
+            c = tuple(v + 0.45 * n for v in center)
+            for d in runs:
+                d.update_body(abi.make_pose(center=c), abi.make_pose(center=c))
+            (fa, ba), (fb, bb) = (d.flags() for d in runs)
+            assert np.array_equal(fa, fb) and np.array_equal(ba, bb), n
+            for x, y in zip(runs[0].links(), runs[1].links()):
+                assert np.array_equal(x, y), n
+            for d in runs:
+                d.step(1)
+        assert rel_l2(runs[0].populations(), runs[1].populations()) <= 6e-6
+    finally:
+        for d in runs:
+            d.close()
