@@ -99,6 +99,13 @@ struct lbm_ctx {
   dim3 grid() const {
     return dim3((unsigned)((g.nx + bx - 1) / bx), (unsigned)((g.ny + by - 1) / by), (unsigned)g.nz);
   }
+  // kernels that only stream a row's nodes (export, initialisation): rows longer than 128 in
+  // blocks of 128 x 1 (FP64 343x220x218 export 435 us, 452 in blocks of 32 x 4 on B200)
+  dim3 row_block() const { return g.nx > 128 ? dim3(128, 1, 1) : block(); }
+  dim3 row_grid() const {
+    const dim3 b = row_block();
+    return dim3((unsigned)((g.nx + b.x - 1) / b.x), (unsigned)((g.ny + b.y - 1) / b.y), (unsigned)g.nz);
+  }
 };
 
 namespace {
@@ -109,14 +116,15 @@ void default_block(lbm_ctx* c) {
   // than 128 take blocks of 128 threads, 32, 64 or 128 wide.  32 x 4 is the fastest wherever
   // faces or the reference step leave work to single lanes (B200, us per step against 128 x 1:
   // FP32 channel 160x96x96 48.6 / 58.5, 384-wide equal, FP64 331x120x119 266 / 278, reference
-  // 480x240x4 26.6 / 28.7); fully periodic boxes take the widest of the three that pads least
-  // (FP32 192x96x96 62.4 / 68.7, FP64 383x120x120 128 x 1 318.7, 32 x 4 322.1).
+  // 480x240x4 26.6 / 28.7); fully periodic boxes and, from 4 M cells, others too take the
+  // widest of the three that pads least (FP32 192x96x96 62.4 / 68.7, FP64 383x120x120 128 x 1
+  // 318.7, 32 x 4 322.1, FP64 channel 225x205x200 549, 32 x 4 580).
   const int nx = c->g.nx;
   int bx = nx <= 128 ? nx : 128;
   if (nx > 128) {
-    const bool periodic = !c->ref && c->g.per[0] && c->g.per[1] && c->g.per[2];
+    const bool widest = !c->ref && ((c->g.per[0] && c->g.per[1] && c->g.per[2]) || c->g.N >= 4000000);
     for (int w : {64, 32})
-      if (!periodic || (nx + w - 1) / w * w < (nx + bx - 1) / bx * bx) bx = w;
+      if (!widest || (nx + w - 1) / w * w < (nx + bx - 1) / bx * bx) bx = w;
   }
   int by = std::max(1, 128 / bx);
   while ((bx * by) % 32 != 0 && bx * (by + 1) <= 256) by++;
@@ -387,10 +395,10 @@ int export_state(lbm_ctx* c, const ExportOut& out) {
   if (c->ref) {
     RefParams p = ref_params(c, c->kin_last_step, F_SOLID_PREV);
     return c->cuda(ref_launch_export(is_ref_fp64(c), p, c->F[1 - c->ri], c->R[1 - c->ri], c->ref_direct ? 1 : 0,
-                                     c->flags, out, nullptr, c->grid(), c->block(), c->stream),
+                                     c->flags, out, nullptr, c->row_grid(), c->row_block(), c->stream),
                    "export");
   }
-  return c->cuda(aa_launch_export(c->cfg.storage, read_params(c), c->A, c->flags, out, c->grid(), c->block(),
+  return c->cuda(aa_launch_export(c->cfg.storage, read_params(c), c->A, c->flags, out, c->row_grid(), c->row_block(),
                                   c->stream),
                  "export");
 }
@@ -404,7 +412,7 @@ int reduce_state(lbm_ctx* c, double out[2]) {
     RefParams p = ref_params(c, c->kin_last_step, F_SOLID_PREV);
     ExportOut none{};
     rc = c->cuda(ref_launch_export(is_ref_fp64(c), p, c->F[1 - c->ri], c->R[1 - c->ri], c->ref_direct ? 1 : 0,
-                                   c->flags, none, c->scratch, c->grid(), c->block(), c->stream),
+                                   c->flags, none, c->scratch, c->row_grid(), c->row_block(), c->stream),
                  "reduce");
   } else {
     rc = c->cuda(aa_launch_reduce(c->cfg.storage, read_params(c), c->A, c->flags, c->scratch, c->grid(),
@@ -989,16 +997,16 @@ int32_t lbm_init_equilibrium(lbm_ctx* c, const double* rho, const double* u, con
   if (c->ref) {
     for (int a = 0; a < 3; a++) p.uni[a] = 0.0;
     void* S = c->F[1 - c->ri];
-    if (c->cuda(ref_launch_init(is_ref_fp64(c), p, S, c->grid(), c->block(), c->stream), "init")) return LBM_ERR_CUDA;
+    if (c->cuda(ref_launch_init(is_ref_fp64(c), p, S, c->row_grid(), c->row_block(), c->stream), "init")) return LBM_ERR_CUDA;
     RefParams rp = ref_params(c, c->kin_latest, F_SOLID);
     if (c->cuda(ref_launch_prepare(is_ref_fp64(c), c->cfg.collision == LBM_COLL_TRT, rp, S, c->F[c->ri], c->R[c->ri],
-                                   c->grid(), c->block(), c->stream),
+                                   c->row_grid(), c->row_block(), c->stream),
                 "prepare"))
       return LBM_ERR_CUDA;
     c->ref_direct = true;
   } else {
     for (int a = 0; a < 3; a++) p.uni[a] = 0.0;
-    if (c->cuda(aa_launch_init(c->cfg.storage, p, c->A, c->flags, c->grid(), c->block(), c->stream), "init"))
+    if (c->cuda(aa_launch_init(c->cfg.storage, p, c->A, c->flags, c->row_grid(), c->row_block(), c->stream), "init"))
       return LBM_ERR_CUDA;
     c->swapped = false;
   }
@@ -1029,15 +1037,15 @@ int32_t lbm_set_populations(lbm_ctx* c, const void* f, int32_t dtype, int32_t la
   p.f_layout = layout;
   if (c->ref) {
     void* S = c->F[1 - c->ri];
-    if (c->cuda(ref_launch_init(is_ref_fp64(c), p, S, c->grid(), c->block(), c->stream), "import")) return LBM_ERR_CUDA;
+    if (c->cuda(ref_launch_init(is_ref_fp64(c), p, S, c->row_grid(), c->row_block(), c->stream), "import")) return LBM_ERR_CUDA;
     RefParams rp = ref_params(c, c->kin_latest, F_SOLID);
     if (c->cuda(ref_launch_prepare(is_ref_fp64(c), c->cfg.collision == LBM_COLL_TRT, rp, S, c->F[c->ri], c->R[c->ri],
-                                   c->grid(), c->block(), c->stream),
+                                   c->row_grid(), c->row_block(), c->stream),
                 "prepare"))
       return LBM_ERR_CUDA;
     c->ref_direct = true;
   } else {
-    if (c->cuda(aa_launch_init(c->cfg.storage, p, c->A, c->flags, c->grid(), c->block(), c->stream), "import"))
+    if (c->cuda(aa_launch_init(c->cfg.storage, p, c->A, c->flags, c->row_grid(), c->row_block(), c->stream), "import"))
       return LBM_ERR_CUDA;
     c->swapped = false;
   }
@@ -1178,7 +1186,7 @@ int32_t lbm_get_macros(lbm_ctx* c, void* rho, void* u, void* v, void* w, int32_t
   out.w = dev[3];
   int rc;
   if (c->ref)
-    rc = c->cuda(ref_launch_macros(is_ref_fp64(c), c->g, c->R[c->ri], out, c->grid(), c->block(), c->stream), "macros");
+    rc = c->cuda(ref_launch_macros(is_ref_fp64(c), c->g, c->R[c->ri], out, c->row_grid(), c->row_block(), c->stream), "macros");
   else
     rc = export_state(c, out);
   if (rc) return rc;
