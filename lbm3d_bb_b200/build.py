@@ -83,7 +83,7 @@ def build_unet(verbose: bool = False, force: bool = False) -> Path:
     """libunet3d.so: the warm-start network's kernels (separate C ABI, include/unet3d.h)."""
     OBJ.mkdir(exist_ok=True)
     src = CSRC / "unet3d.cu"
-    if force or _stale(UNET_LIB, [src, INCLUDE / "unet3d.h"]):
+    if force or _stale(UNET_LIB, [src, CSRC / "chained.cuh", INCLUDE / "unet3d.h"]):
         cmd = [nvcc(), *ARCH, *COMMON, "-shared", str(src), "-o", str(UNET_LIB), "-lcudart"]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")

@@ -1,6 +1,7 @@
 // lbm_kernels.h — kernel parameter blocks and host launchers of liblbm3d.
 #pragma once
 
+#include "chained.cuh"
 #include "lbm_internal.cuh"
 
 namespace lbm {
@@ -229,31 +230,6 @@ __device__ __forceinline__ void block_force_reduce(double* acc, bool has, double
       atomicAdd(out + k, s);
     }
   }
-}
-
-// Chained launches.  A kernel of the time loop begins with chain_begin(): the next kernel of the
-// stream, launched with launch_chained, may then be placed on the SMs as soon as every block
-// here has started, and waits in its own chain_begin() until this one has completed and its
-// writes are visible.  That hides the launch latency and the ramp between dependent kernels
-// (B200, us per step: channel 96x48x48 11.4 -> 9.4, 192x96x96 TRT 60.4 -> 58.4, reference
-// 480x240x4 26.8 -> 25.2).  Launched any other way, chain_begin() does nothing.
-__device__ __forceinline__ void chain_begin() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-template <class... P, class... A>
-inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A&&... args) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.stream = s;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
 // ---- launchers (kernels_aa.cu; kernels in aa_impl.cuh) ----

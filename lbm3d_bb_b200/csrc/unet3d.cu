@@ -30,6 +30,12 @@
 #include <type_traits>
 
 #include "../../include/unet3d.h"
+#include "chained.cuh"
+
+using lbm::chain_begin;
+using lbm::chain_trigger;
+using lbm::chain_wait;
+using lbm::launch_chained_smem;  // (kernel, grid, block, dynamic shared memory, stream, arguments...)
 
 namespace {
 
@@ -83,6 +89,7 @@ __global__ void __launch_bounds__(128) conv_fwd_kernel(const bf16* __restrict__ 
                                                        const float* __restrict__ bias, bf16* __restrict__ out,
                                                        const Geo g, const int cin, const int relu,
                                                        const long long tiles) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const long long tile = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (tile >= tiles) return;  // whole warp
@@ -205,6 +212,7 @@ __device__ __forceinline__ bool tc_mbar_wait(uint64_t* bar, uint32_t parity, int
 // MMA commits to it and nothing arrives, so the wait gives up after `polls` polls and
 // the block sets the error word as a convolution CTA does.  Nothing is in flight.
 __global__ void __launch_bounds__(32) tc_wait_probe_kernel(const int polls, int* err) {
+  chain_begin();
   __shared__ __align__(8) uint64_t bar;
   if (threadIdx.x == 0) {
     tc_mbar_init(&bar);
@@ -369,6 +377,9 @@ __global__ void __launch_bounds__(HT_THREADS, 1)
     tc_mbar_init(&bar[1]);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  __syncthreads();  // the columns are ours
+  chain_trigger();
+  chain_wait();
   for (int c = tid; c < COUT; c += HT_THREADS) sbias[c] = bias ? bias[c] : 0.f;
   const int first = blockIdx.x, stride = gridDim.x;
   const int mine = (a.tiles - first + stride - 1) / stride;
@@ -571,6 +582,8 @@ __global__ void __launch_bounds__(TC_M) conv_fwd_tma_kernel(const __grid_constan
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  chain_trigger();
+  chain_wait();
   const uint32_t tmem = tmem_base;
   // tile -> (n, z, y0, x0): 128 voxels = part of one row (W >= 128) or 128/W whole rows
   const int bw = g.w < TC_M ? g.w : TC_M, bh = TC_M / bw;
@@ -669,6 +682,7 @@ __global__ void __launch_bounds__(TC_M) conv_fwd_tma_kernel(const __grid_constan
 
 // wt[26 - tap][ci][co] = w[tap][co][ci]
 __global__ void flip_kernel(const bf16* __restrict__ w, bf16* __restrict__ wt, int cin, int cout) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int total = 27 * cin * cout;
   if (i >= total) return;
@@ -683,6 +697,7 @@ template <int CB>  // output channels / 16 (1, 2 or 4)
 __global__ void __launch_bounds__(128) conv_bwdw_kernel(const bf16* __restrict__ in, const bf16* __restrict__ dout,
                                                         float* __restrict__ dw, const Geo g, const int cin,
                                                         const long long vox, const long long chunk) {
+  chain_begin();
   constexpr int COUT = CB * 16;
   constexpr int SA = COUT + 8, SB = 16 + 8;  // padded row lengths (16-byte multiples)
   __shared__ __align__(16) bf16 sA[BW_KV * SA];
@@ -816,6 +831,8 @@ __global__ void __launch_bounds__(BT_THREADS, 1)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  chain_trigger();
+  chain_wait();
   const uint32_t tmem = tmem_base;
   const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
   for (int c = (warp >> 2) * 16; c < BUFS * COLS; c += 32) tc_zero16(lanes + c);  // every MMA accumulates
@@ -970,6 +987,7 @@ __global__ void __launch_bounds__(BT_THREADS, 1)
 }
 
 __global__ void bias_grad_kernel(const bf16* __restrict__ dout, float* __restrict__ db, long long voxels, int c) {
+  chain_begin();
   extern __shared__ float sacc[];
   for (int k = threadIdx.x; k < c; k += blockDim.x) sacc[k] = 0.f;
   __syncthreads();
@@ -1029,6 +1047,7 @@ __device__ __forceinline__ Row row_of(long long r, int d, int h) {
 }
 
 __global__ void bias_grad8_kernel(const bf16* __restrict__ dout, float* __restrict__ db, long long groups, int c) {
+  chain_begin();
   extern __shared__ float sacc[];
   for (int k = threadIdx.x; k < c; k += blockDim.x) sacc[k] = 0.f;
   __syncthreads();
@@ -1064,6 +1083,7 @@ __device__ __forceinline__ uint32_t relu_mask2(uint32_t dy, uint32_t y) {  // tw
   return (lo > 0.f ? dy & 0xffffu : 0u) | (hi > 0.f ? dy & 0xffff0000u : 0u);
 }
 __global__ void relu_bwd8_kernel(uint4* __restrict__ dy, const uint4* __restrict__ y, long long groups) {
+  chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= groups) return;
   const uint4 g = dy[i], v = __ldg(y + i);
@@ -1071,6 +1091,7 @@ __global__ void relu_bwd8_kernel(uint4* __restrict__ dy, const uint4* __restrict
 }
 
 __global__ void pool2x8_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, Geo f, int c) {
+  chain_begin();
   const int W = f.w / 2, gc = c / 8;
   const Row q = row_of(blockIdx.x, f.d / 2, f.h / 2);
   for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < W * gc; i += gridDim.y * blockDim.x) {
@@ -1090,6 +1111,7 @@ __global__ void pool2x8_kernel(const bf16* __restrict__ in, bf16* __restrict__ o
 }
 
 __global__ void pool2x8_bwd_kernel(const bf16* __restrict__ dout, bf16* __restrict__ din, Geo f, int c, int accumulate) {
+  chain_begin();
   const int gc = c / 8;
   const Row q = row_of(blockIdx.x, f.d, f.h);
   const long long parent = ((q.n * (f.d / 2) + q.z / 2) * (f.h / 2) + q.y / 2) * (f.w / 2);
@@ -1114,6 +1136,7 @@ __global__ void pool2x8_bwd_kernel(const bf16* __restrict__ dout, bf16* __restri
 
 __global__ void up2_concat8_kernel(const uint4* __restrict__ low, const uint4* __restrict__ skip,
                                    uint4* __restrict__ out, Geo f, int gu, int gs) {
+  chain_begin();
   const int gt = gu + gs;
   const Row q = row_of(blockIdx.x, f.d, f.h);
   const long long parent = ((q.n * (f.d / 2) + q.z / 2) * (f.h / 2) + q.y / 2) * (f.w / 2);
@@ -1126,6 +1149,7 @@ __global__ void up2_concat8_kernel(const uint4* __restrict__ low, const uint4* _
 
 __global__ void up2_concat8_bwd_kernel(const bf16* __restrict__ dcat, bf16* __restrict__ dlow, uint4* __restrict__ dskip,
                                        Geo f, int gu, int gs, unsigned coarse_rows) {
+  chain_begin();
   const int ct = (gu + gs) * 8;
   if (blockIdx.x < coarse_rows) {  // dlow: the 8 children of a coarse voxel
     const int W = f.w / 2;
@@ -1153,12 +1177,14 @@ __global__ void up2_concat8_bwd_kernel(const bf16* __restrict__ dcat, bf16* __re
 }
 
 __global__ void relu_bwd_kernel(bf16* __restrict__ dy, const bf16* __restrict__ y, long long count) {
+  chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count && !(__bfloat162float(y[i]) > 0.f)) dy[i] = __float2bfloat16(0.f);
 }
 
 // ---- pooling, upsampling, concatenation ---------------------------------------------
 __global__ void pool2_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, Geo f, int c, long long count) {
+  chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;  // count = coarse elements
   const int ch = (int)(i % c);
@@ -1181,6 +1207,7 @@ __global__ void pool2_kernel(const bf16* __restrict__ in, bf16* __restrict__ out
 
 __global__ void pool2_bwd_kernel(const bf16* __restrict__ dout, bf16* __restrict__ din, Geo f, int c, int accumulate,
                                  long long count) {
+  chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;  // count = fine elements
   const int ch = (int)(i % c);
@@ -1199,6 +1226,7 @@ __global__ void pool2_bwd_kernel(const bf16* __restrict__ dout, bf16* __restrict
 
 __global__ void up2_concat_kernel(const bf16* __restrict__ low, const bf16* __restrict__ skip, bf16* __restrict__ out,
                                   Geo f, int cu, int cs, long long count) {
+  chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;  // count = fine voxels * (cu + cs)
   const int ct = cu + cs;
@@ -1221,6 +1249,7 @@ __global__ void up2_concat_kernel(const bf16* __restrict__ low, const bf16* __re
 
 __global__ void up2_concat_bwd_low_kernel(const bf16* __restrict__ dcat, bf16* __restrict__ dlow, Geo f, int cu, int cs,
                                           long long count) {
+  chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;  // count = coarse voxels * cu
   const int ch = (int)(i % cu);
@@ -1243,6 +1272,7 @@ __global__ void up2_concat_bwd_low_kernel(const bf16* __restrict__ dcat, bf16* _
 
 __global__ void up2_concat_bwd_skip_kernel(const bf16* __restrict__ dcat, bf16* __restrict__ dskip, int cu, int cs,
                                            long long count) {
+  chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;  // count = fine voxels * cs
   const long long v = i / cs;
@@ -1258,6 +1288,7 @@ __global__ void __launch_bounds__(256) mse_kernel(const bf16* __restrict__ out, 
                                                   const uint8_t* __restrict__ mask, const float* __restrict__ cw,
                                                   bf16* __restrict__ dout, double* loss, long long voxels, int cpad,
                                                   int ct, double count) {
+  chain_begin();
   __shared__ double part[8];
   double l = 0.0;
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < voxels; v += (long long)gridDim.x * blockDim.x) {
@@ -1307,6 +1338,7 @@ __global__ void __launch_bounds__(256) mse_kernel(const bf16* __restrict__ out, 
 __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
                             float* __restrict__ v, bf16* __restrict__ wb, long long count, float lr, float b1, float b2,
                             float eps, float c1, float c2) {
+  chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const float gi = g[i];
@@ -1320,11 +1352,13 @@ __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, 
 }
 
 __global__ void to_bf16_kernel(const float* __restrict__ x, bf16* __restrict__ y, long long count) {
+  chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) y[i] = __float2bfloat16(x[i]);
 }
 
 __global__ void from_bf16_kernel(const bf16* __restrict__ x, float* __restrict__ y, long long count) {
+  chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) y[i] = __bfloat162float(x[i]);
 }
@@ -1332,6 +1366,7 @@ __global__ void from_bf16_kernel(const bf16* __restrict__ x, float* __restrict__
 // out[0] += sum (a - b)^2, out[1] += sum a^2 (FP64), for steady-state tests.
 __global__ void diff_norms_kernel(const float* __restrict__ a, const float* __restrict__ b, long long count,
                                   double* out) {
+  chain_begin();
   double d2 = 0.0, a2 = 0.0;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x) {
     const double x = a[i], y = b[i];
@@ -1359,6 +1394,7 @@ struct Ellipsoid {
 // node position; the mask uses the solver's rasteriser expression with unfused
 // FP64 operations, so it matches the solver's solid flags.
 __global__ void features_kernel(bf16* __restrict__ out, int nx, int ny, int nz, Ellipsoid e, float re_feature) {
+  chain_begin();
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long n = (long long)nx * ny * nz;
   if (v >= n) return;
@@ -1402,6 +1438,7 @@ __global__ void features_kernel(bf16* __restrict__ out, int nx, int ny, int nz, 
 // (channel 2 = u_y, 3 = u_z) negated: undoes a reflection of the input.
 __global__ void unpack_fields_kernel(const bf16* __restrict__ y, float* __restrict__ out, Geo g, int flip_y, int flip_z,
                                      float weight, int accumulate, long long count) {
+  chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;  // count = n * d * h * w
   long long t = i;
@@ -1566,7 +1603,7 @@ int halo_launch(const bf16* in, const bf16* w, const float* bias, bf16* out, con
                 cudaStream_t s) {
   static std::atomic<unsigned long long> done{0};
   if (!allow_smem(conv_halo_kernel<COUT, BX>, HT_MAX_SMEM, done)) return launched("nn_conv3d_fwd (shared memory)");
-  conv_halo_kernel<COUT, BX><<<p.grid, HT_THREADS, p.smem, s>>>(in, w, bias, out, p.a, err);
+  launch_chained_smem(conv_halo_kernel<COUT, BX>, p.grid, HT_THREADS, p.smem, s, in, w, bias, out, p.a, err);
   return launched("nn_conv3d_fwd (tcgen05)");
 }
 
@@ -1663,7 +1700,7 @@ int bw_launch(const bf16* in, const bf16* dout, float* dw, const Geo& g, int cin
       !activation_map(ymap, dout, g, cout, false, 16, p.a.bp, CO / 8))
     return 0;
   if (!allow_smem(conv_bwdw_tc_kernel<CI, CO>, BT_MAX_SMEM, allowed)) return launched("nn_conv3d_bwd_weight") ? -1 : 0;
-  conv_bwdw_tc_kernel<CI, CO><<<p.grid, BT_THREADS, p.smem, s>>>(xmap, ymap, dw, p.a, err);
+  launch_chained_smem(conv_bwdw_tc_kernel<CI, CO>, p.grid, BT_THREADS, p.smem, s, xmap, ymap, dw, p.a, err);
   return launched("nn_conv3d_bwd_weight (tcgen05)") ? -1 : 1;
 }
 
@@ -1722,11 +1759,16 @@ int32_t nn_conv3d_fwd(const void* in, const void* w, const float* bias, void* ou
       if (r1 != CUDA_SUCCESS || r2 != CUDA_SUCCESS) return fail("nn_conv3d_fwd: tensor map encoding failed (%d, %d)", (int)r1, (int)r2);
       const unsigned tgrid = (unsigned)((long long)n * d * (h / (TC_M / bw)) * (wd / bw));
       switch (cout) {
-        case 16: conv_fwd_tma_kernel<16><<<tgrid, TC_M, 0, s>>>(xmap, wmap, bias, O, g, cin, relu, err); break;
-        case 32: conv_fwd_tma_kernel<32><<<tgrid, TC_M, 0, s>>>(xmap, wmap, bias, O, g, cin, relu, err); break;
-        case 48: conv_fwd_tma_kernel<48><<<tgrid, TC_M, 0, s>>>(xmap, wmap, bias, O, g, cin, relu, err); break;
-        case 64: conv_fwd_tma_kernel<64><<<tgrid, TC_M, 0, s>>>(xmap, wmap, bias, O, g, cin, relu, err); break;
-        case 96: conv_fwd_tma_kernel<96><<<tgrid, TC_M, 0, s>>>(xmap, wmap, bias, O, g, cin, relu, err); break;
+        case 16: launch_chained_smem(conv_fwd_tma_kernel<16>, tgrid, TC_M, 0, s, xmap, wmap, bias, O, g, cin, relu,
+                                     err); break;
+        case 32: launch_chained_smem(conv_fwd_tma_kernel<32>, tgrid, TC_M, 0, s, xmap, wmap, bias, O, g, cin, relu,
+                                     err); break;
+        case 48: launch_chained_smem(conv_fwd_tma_kernel<48>, tgrid, TC_M, 0, s, xmap, wmap, bias, O, g, cin, relu,
+                                     err); break;
+        case 64: launch_chained_smem(conv_fwd_tma_kernel<64>, tgrid, TC_M, 0, s, xmap, wmap, bias, O, g, cin, relu,
+                                     err); break;
+        case 96: launch_chained_smem(conv_fwd_tma_kernel<96>, tgrid, TC_M, 0, s, xmap, wmap, bias, O, g, cin, relu,
+                                     err); break;
         default: return fail("nn_conv3d_fwd: Cout %d not in {16, 32, 48, 64, 96}", cout);
       }
       return launched("nn_conv3d_fwd (tcgen05, TMA)");
@@ -1743,11 +1785,11 @@ int32_t nn_conv3d_fwd(const void* in, const void* w, const float* bias, void* ou
     }
   }
   switch (cout) {
-    case 16: conv_fwd_kernel<2><<<grid, 128, 0, s>>>(I, W, bias, O, g, cin, relu, tiles); break;
-    case 32: conv_fwd_kernel<4><<<grid, 128, 0, s>>>(I, W, bias, O, g, cin, relu, tiles); break;
-    case 48: conv_fwd_kernel<6><<<grid, 128, 0, s>>>(I, W, bias, O, g, cin, relu, tiles); break;
-    case 64: conv_fwd_kernel<8><<<grid, 128, 0, s>>>(I, W, bias, O, g, cin, relu, tiles); break;
-    case 96: conv_fwd_kernel<12><<<grid, 128, 0, s>>>(I, W, bias, O, g, cin, relu, tiles); break;
+    case 16: launch_chained_smem(conv_fwd_kernel<2>, grid, 128, 0, s, I, W, bias, O, g, cin, relu, tiles); break;
+    case 32: launch_chained_smem(conv_fwd_kernel<4>, grid, 128, 0, s, I, W, bias, O, g, cin, relu, tiles); break;
+    case 48: launch_chained_smem(conv_fwd_kernel<6>, grid, 128, 0, s, I, W, bias, O, g, cin, relu, tiles); break;
+    case 64: launch_chained_smem(conv_fwd_kernel<8>, grid, 128, 0, s, I, W, bias, O, g, cin, relu, tiles); break;
+    case 96: launch_chained_smem(conv_fwd_kernel<12>, grid, 128, 0, s, I, W, bias, O, g, cin, relu, tiles); break;
     default: return fail("nn_conv3d_fwd: Cout %d not in {16, 32, 48, 64, 96}", cout);
   }
   return launched("nn_conv3d_fwd");
@@ -1788,7 +1830,7 @@ int32_t nn_wait_selftest(int32_t polls, void* stream) {
   if (polls < 1 || polls > TC_WAIT_POLLS) return fail("nn_wait_selftest: polls %d outside [1, %d]", polls, TC_WAIT_POLLS);
   int* err = tc_err_ptr();
   if (!err) return fail("nn_wait_selftest: no device address for the error word");
-  tc_wait_probe_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(polls, err);
+  launch_chained_smem(tc_wait_probe_kernel, 1, 32, 0, (cudaStream_t)stream, polls, err);
   const int rc = launched("nn_wait_selftest");
   if (rc) return rc;
   return nn_tc_status(stream);
@@ -1797,7 +1839,8 @@ int32_t nn_wait_selftest(int32_t polls, void* stream) {
 int32_t nn_conv3d_flip(const void* w, void* wt, int32_t cin, int32_t cout, void* stream) {
   if (!w || !wt || cin <= 0 || cout <= 0) return fail("nn_conv3d_flip: bad arguments");
   const int total = 27 * cin * cout;
-  flip_kernel<<<blocks_for(total, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)w, (bf16*)wt, cin, cout);
+  launch_chained_smem(flip_kernel, blocks_for(total, 256), 256, 0, (cudaStream_t)stream, (const bf16*)w, (bf16*)wt,
+                      cin, cout);
   return launched("nn_conv3d_flip");
 }
 
@@ -1821,9 +1864,9 @@ int32_t nn_conv3d_bwd_weight(const void* in, const void* dout, float* dw, int32_
     if (rc) return rc < 0 ? 1 : 0;
   }
   switch (cout) {
-    case 16: conv_bwdw_kernel<1><<<grid, 128, 0, s>>>(I, D, dw, g, cin, vox, chunk); break;
-    case 32: conv_bwdw_kernel<2><<<grid, 128, 0, s>>>(I, D, dw, g, cin, vox, chunk); break;
-    case 64: conv_bwdw_kernel<4><<<grid, 128, 0, s>>>(I, D, dw, g, cin, vox, chunk); break;
+    case 16: launch_chained_smem(conv_bwdw_kernel<1>, grid, 128, 0, s, I, D, dw, g, cin, vox, chunk); break;
+    case 32: launch_chained_smem(conv_bwdw_kernel<2>, grid, 128, 0, s, I, D, dw, g, cin, vox, chunk); break;
+    case 64: launch_chained_smem(conv_bwdw_kernel<4>, grid, 128, 0, s, I, D, dw, g, cin, vox, chunk); break;
     default: return fail("nn_conv3d_bwd_weight: Cout %d not in {16, 32, 64}", cout);
   }
   return launched("nn_conv3d_bwd_weight");
@@ -1835,13 +1878,15 @@ int32_t nn_bias_grad(const void* dout, float* db, int64_t voxels, int32_t c, voi
     const long long groups = voxels * (c / 8);
     unsigned grid = blocks_for(groups, 256 * 4);
     if (grid > 1184u) grid = 1184u;  // eight blocks on each of 148 SMs: 14 groups a thread at 2 M voxels
-    bias_grad8_kernel<<<grid, 256, c * sizeof(float), (cudaStream_t)stream>>>((const bf16*)dout, db, groups, c);
+    launch_chained_smem(bias_grad8_kernel, grid, 256, c * sizeof(float), (cudaStream_t)stream, (const bf16*)dout, db,
+                        groups, c);
     return launched("nn_bias_grad");
   }
   const long long total = voxels * c;
   unsigned grid = blocks_for(total, 256 * 16);
   if (grid > 4096) grid = 4096;
-  bias_grad_kernel<<<grid, 256, c * sizeof(float), (cudaStream_t)stream>>>((const bf16*)dout, db, voxels, c);
+  launch_chained_smem(bias_grad_kernel, grid, 256, c * sizeof(float), (cudaStream_t)stream, (const bf16*)dout, db,
+                      voxels, c);
   return launched("nn_bias_grad");
 }
 
@@ -1849,10 +1894,12 @@ int32_t nn_relu_bwd(void* dy, const void* y, int64_t count, void* stream) {
   if (!dy || !y || count < 0) return fail("nn_relu_bwd: bad arguments");
   if (count == 0) return 0;
   if (count % 8 == 0 && aligned16(dy) && aligned16(y)) {
-    relu_bwd8_kernel<<<blocks_for(count / 8, 256), 256, 0, (cudaStream_t)stream>>>((uint4*)dy, (const uint4*)y, count / 8);
+    launch_chained_smem(relu_bwd8_kernel, blocks_for(count / 8, 256), 256, 0, (cudaStream_t)stream, (uint4*)dy,
+                        (const uint4*)y, count / 8);
     return launched("nn_relu_bwd");
   }
-  relu_bwd_kernel<<<blocks_for(count, 256), 256, 0, (cudaStream_t)stream>>>((bf16*)dy, (const bf16*)y, count);
+  launch_chained_smem(relu_bwd_kernel, blocks_for(count, 256), 256, 0, (cudaStream_t)stream, (bf16*)dy,
+                      (const bf16*)y, count);
   return launched("nn_relu_bwd");
 }
 
@@ -1860,12 +1907,13 @@ int32_t nn_pool2(const void* in, void* out, int32_t n, int32_t d, int32_t h, int
   if (!in || !out || !geo_ok(n, d, h, wd) || c <= 0 || d % 2 || h % 2 || wd % 2) return fail("nn_pool2: bad shape");
   const long long rows = (long long)n * (d / 2) * (h / 2);
   if (grouped(c, rows, in, out)) {
-    pool2x8_kernel<<<row_grid(rows, wd / 2 * (c / 8)), 256, 0, (cudaStream_t)stream>>>((const bf16*)in, (bf16*)out,
+    launch_chained_smem(pool2x8_kernel, row_grid(rows, wd / 2 * (c / 8)), 256, 0, (cudaStream_t)stream,
+                        (const bf16*)in, (bf16*)out,
                                                                                        Geo{n, d, h, wd}, c);
     return launched("nn_pool2");
   }
   const long long count = (long long)n * (d / 2) * (h / 2) * (wd / 2) * c;
-  pool2_kernel<<<blocks_for(count, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)in, (bf16*)out,
+  launch_chained_smem(pool2_kernel, blocks_for(count, 256), 256, 0, (cudaStream_t)stream, (const bf16*)in, (bf16*)out,
                                                                           Geo{n, d, h, wd}, c, count);
   return launched("nn_pool2");
 }
@@ -1875,12 +1923,14 @@ int32_t nn_pool2_bwd(const void* dout, void* din, int32_t n, int32_t d, int32_t 
   if (!dout || !din || !geo_ok(n, d, h, wd) || c <= 0 || d % 2 || h % 2 || wd % 2) return fail("nn_pool2_bwd: bad shape");
   const long long rows = (long long)n * d * h;
   if (grouped(c, rows, dout, din)) {
-    pool2x8_bwd_kernel<<<row_grid(rows, wd * (c / 8)), 256, 0, (cudaStream_t)stream>>>((const bf16*)dout, (bf16*)din,
+    launch_chained_smem(pool2x8_bwd_kernel, row_grid(rows, wd * (c / 8)), 256, 0, (cudaStream_t)stream,
+                        (const bf16*)dout, (bf16*)din,
                                                                                        Geo{n, d, h, wd}, c, accumulate);
     return launched("nn_pool2_bwd");
   }
   const long long count = (long long)n * d * h * wd * c;
-  pool2_bwd_kernel<<<blocks_for(count, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)dout, (bf16*)din,
+  launch_chained_smem(pool2_bwd_kernel, blocks_for(count, 256), 256, 0, (cudaStream_t)stream, (const bf16*)dout,
+                      (bf16*)din,
                                                                               Geo{n, d, h, wd}, c, accumulate, count);
   return launched("nn_pool2_bwd");
 }
@@ -1891,13 +1941,13 @@ int32_t nn_up2_concat(const void* low, const void* skip, void* out, int32_t n, i
     return fail("nn_up2_concat: bad shape");
   const long long rows = (long long)n * d * h;
   if (cu % 8 == 0 && grouped(cs, rows, low, skip, out)) {
-    up2_concat8_kernel<<<row_grid(rows, wd * ((cu + cs) / 8)), 256, 0, (cudaStream_t)stream>>>(
-        (const uint4*)low, (const uint4*)skip, (uint4*)out, Geo{n, d, h, wd}, cu / 8, cs / 8);
+    launch_chained_smem(up2_concat8_kernel, row_grid(rows, wd * ((cu + cs) / 8)), 256, 0, (cudaStream_t)stream,
+                        (const uint4*)low, (const uint4*)skip, (uint4*)out, Geo{n, d, h, wd}, cu / 8, cs / 8);
     return launched("nn_up2_concat");
   }
   const long long count = (long long)n * d * h * wd * (cu + cs);
-  up2_concat_kernel<<<blocks_for(count, 256), 256, 0, (cudaStream_t)stream>>>(
-      (const bf16*)low, (const bf16*)skip, (bf16*)out, Geo{n, d, h, wd}, cu, cs, count);
+  launch_chained_smem(up2_concat_kernel, blocks_for(count, 256), 256, 0, (cudaStream_t)stream, (const bf16*)low,
+                      (const bf16*)skip, (bf16*)out, Geo{n, d, h, wd}, cu, cs, count);
   return launched("nn_up2_concat");
 }
 
@@ -1909,15 +1959,18 @@ int32_t nn_up2_concat_bwd(const void* dcat, void* dlow, void* dskip, int32_t n, 
   const long long coarse = (long long)n * (d / 2) * (h / 2), rows = coarse + (long long)n * d * h;
   if (cu % 8 == 0 && grouped(cs, rows, dcat, dlow, dskip)) {
     const int per_row = wd / 2 * (cu / 8) > wd * (cs / 8) ? wd / 2 * (cu / 8) : wd * (cs / 8);
-    up2_concat8_bwd_kernel<<<row_grid(rows, per_row), 256, 0, s>>>((const bf16*)dcat, (bf16*)dlow, (uint4*)dskip,
+    launch_chained_smem(up2_concat8_bwd_kernel, row_grid(rows, per_row), 256, 0, s, (const bf16*)dcat, (bf16*)dlow,
+                        (uint4*)dskip,
                                                                    Geo{n, d, h, wd}, cu / 8, cs / 8, (unsigned)coarse);
     return launched("nn_up2_concat_bwd");
   }
   const long long cl = (long long)n * (d / 2) * (h / 2) * (wd / 2) * cu;
-  up2_concat_bwd_low_kernel<<<blocks_for(cl, 256), 256, 0, s>>>((const bf16*)dcat, (bf16*)dlow, Geo{n, d, h, wd}, cu,
+  launch_chained_smem(up2_concat_bwd_low_kernel, blocks_for(cl, 256), 256, 0, s, (const bf16*)dcat, (bf16*)dlow,
+                      Geo{n, d, h, wd}, cu,
                                                                  cs, cl);
   const long long cf = (long long)n * d * h * wd * cs;
-  up2_concat_bwd_skip_kernel<<<blocks_for(cf, 256), 256, 0, s>>>((const bf16*)dcat, (bf16*)dskip, cu, cs, cf);
+  launch_chained_smem(up2_concat_bwd_skip_kernel, blocks_for(cf, 256), 256, 0, s, (const bf16*)dcat, (bf16*)dskip, cu,
+                      cs, cf);
   return launched("nn_up2_concat_bwd");
 }
 
@@ -1928,7 +1981,8 @@ int32_t nn_mse(const void* out, const float* target, const uint8_t* mask, const 
   const unsigned grid = blocks_for(voxels, 256) < 1184u ? blocks_for(voxels, 256) : 1184u;
   const auto kernel = cpad == 16 && ct == 4 && aligned16(out) && aligned16(target) && aligned16(dout) ? mse_kernel<true>
                                                                                                      : mse_kernel<false>;
-  kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const bf16*)out, target, mask, cw, (bf16*)dout, loss, voxels, cpad, ct,
+  launch_chained_smem(kernel, grid, 256, 0, (cudaStream_t)stream, (const bf16*)out, target, mask, cw, (bf16*)dout,
+                      loss, voxels, cpad, ct,
                                                  count);
   return launched("nn_mse");
 }
@@ -1938,7 +1992,8 @@ int32_t nn_adam(float* w, const float* g, float* m, float* v, void* wb, int64_t 
   if (!w || !g || !m || !v || count < 0 || t < 1) return fail("nn_adam: bad arguments");
   if (count == 0) return 0;
   const float c1 = 1.f - powf(beta1, (float)t), c2 = 1.f - powf(beta2, (float)t);
-  adam_kernel<<<blocks_for(count, 256), 256, 0, (cudaStream_t)stream>>>(w, g, m, v, (bf16*)wb, count, lr, beta1, beta2,
+  launch_chained_smem(adam_kernel, blocks_for(count, 256), 256, 0, (cudaStream_t)stream, w, g, m, v, (bf16*)wb, count,
+                      lr, beta1, beta2,
                                                                          eps, c1, c2);
   return launched("nn_adam");
 }
@@ -1948,7 +2003,7 @@ int32_t nn_diff_norms(const float* a, const float* b, int64_t count, double* out
   if (count == 0) return 0;
   unsigned grid = blocks_for(count, 256 * 8);
   if (grid > 2048) grid = 2048;
-  diff_norms_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(a, b, count, out);
+  launch_chained_smem(diff_norms_kernel, grid, 256, 0, (cudaStream_t)stream, a, b, count, out);
   return launched("nn_diff_norms");
 }
 
@@ -1962,7 +2017,8 @@ int32_t nn_features_ellipsoid(void* out, int32_t nx, int32_t ny, int32_t nz, con
   }
   for (int k = 0; k < 9; k++) e.rot[k] = rot[k];
   const long long n = (long long)nx * ny * nz;
-  features_kernel<<<blocks_for(n, 256), 256, 0, (cudaStream_t)stream>>>((bf16*)out, nx, ny, nz, e, re_feature);
+  launch_chained_smem(features_kernel, blocks_for(n, 256), 256, 0, (cudaStream_t)stream, (bf16*)out, nx, ny, nz, e,
+                      re_feature);
   return launched("nn_features_ellipsoid");
 }
 
@@ -1970,22 +2026,22 @@ int32_t nn_unpack_fields(const void* y, float* out, int32_t n, int32_t d, int32_
                          int32_t flip_z, float weight, int32_t accumulate, void* stream) {
   if (!y || !out || !geo_ok(n, d, h, wd)) return fail("nn_unpack_fields: bad arguments");
   const long long count = (long long)n * d * h * wd;
-  unpack_fields_kernel<<<blocks_for(count, 256), 256, 0, (cudaStream_t)stream>>>(
-      (const bf16*)y, out, Geo{n, d, h, wd}, flip_y, flip_z, weight, accumulate, count);
+  launch_chained_smem(unpack_fields_kernel, blocks_for(count, 256), 256, 0, (cudaStream_t)stream, (const bf16*)y, out,
+                      Geo{n, d, h, wd}, flip_y, flip_z, weight, accumulate, count);
   return launched("nn_unpack_fields");
 }
 
 int32_t nn_to_bf16(const float* x, void* y, int64_t count, void* stream) {
   if (!x || !y || count < 0) return fail("nn_to_bf16: bad arguments");
   if (count == 0) return 0;
-  to_bf16_kernel<<<blocks_for(count, 256), 256, 0, (cudaStream_t)stream>>>(x, (bf16*)y, count);
+  launch_chained_smem(to_bf16_kernel, blocks_for(count, 256), 256, 0, (cudaStream_t)stream, x, (bf16*)y, count);
   return launched("nn_to_bf16");
 }
 
 int32_t nn_from_bf16(const void* x, float* y, int64_t count, void* stream) {
   if (!x || !y || count < 0) return fail("nn_from_bf16: bad arguments");
   if (count == 0) return 0;
-  from_bf16_kernel<<<blocks_for(count, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, y, count);
+  launch_chained_smem(from_bf16_kernel, blocks_for(count, 256), 256, 0, (cudaStream_t)stream, (const bf16*)x, y, count);
   return launched("nn_from_bf16");
 }
 
