@@ -212,16 +212,34 @@ class UNet3D:
         self.layers = layer_table(width)
         src = params if params is not None else init_params(width, seed)
         f32 = dict(dtype=torch.float32, device=self.dev)
-        self.W = {k: torch.from_numpy(np.ascontiguousarray(v, np.float32)).to(**f32) for k, v in src.items()}
-        self.Wb = {}
+        # every parameter is a view of one flat buffer (as are its gradient, moments and BF16
+        # copy), so the optimiser and zero_grad are one launch each instead of one per tensor
+        sizes = {k: (int(np.size(v)) + 7) // 8 * 8 for k, v in src.items()}  # 16-byte aligned in BF16
+        total = sum(sizes.values())
+        self._flat = {n: torch.zeros(total, **f32) for n in "WGMV"}
+        self._flat["Wb"] = torch.empty(total, dtype=torch.bfloat16, device=self.dev)
+        views: dict[str, dict] = {n: {} for n in self._flat}
+        at = 0
+        for k, v in src.items():
+            v = np.ascontiguousarray(v, np.float32)
+            for n, buf in self._flat.items():
+                views[n][k] = buf[at:at + v.size].view(v.shape)
+            views["W"][k].copy_(torch.from_numpy(v))
+            at += sizes[k]
+        self.W, self.G, self.M, self.V = (views[n] for n in "WGMV")
+        self.Wb = {name: views["Wb"][f"{name}.w"] for name, _, _, _ in self.layers}
         for name, cin, cout, _ in self.layers:
-            self.Wb[name] = torch.empty((27, cout, cin), dtype=torch.bfloat16, device=self.dev)
             self.ops.to_bf16(self.W[f"{name}.w"], self.Wb[name])
-        self.G = {k: torch.zeros_like(v) for k, v in self.W.items()}
-        self.M = {k: torch.zeros_like(v) for k, v in self.W.items()}
-        self.V = {k: torch.zeros_like(v) for k, v in self.W.items()}
+        self._views = {(n, k): t.data_ptr() for n, d in self._named() for k, t in d.items()}
         self.t = 0
         self._shape = None
+
+    def _named(self):
+        return (("W", self.W), ("G", self.G), ("M", self.M), ("V", self.V), ("Wb", self.Wb))
+
+    def _whole(self, *names) -> bool:
+        """True while the tensors of these groups are the views of the flat buffers."""
+        return all(self._views.get((n, k)) == t.data_ptr() for n, d in self._named() if n in names for k, t in d.items())
 
     # -- buffers -----------------------------------------------------------------------
     def _alloc(self, shape):
@@ -306,6 +324,9 @@ class UNet3D:
         self._back("e1a", A["x"], D["a1"], None, 1, A["a1"])
 
     def zero_grad(self):
+        if self._whole("G"):
+            self._flat["G"].zero_()
+            return
         for g in self.G.values():
             g.zero_()
 
@@ -322,6 +343,10 @@ class UNet3D:
 
     def adam_step(self, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
         self.t += 1
+        if self._whole("W", "G", "M", "V", "Wb"):
+            f = self._flat
+            self.ops.adam(f["W"], f["G"], f["M"], f["V"], f["Wb"], lr, b1, b2, eps, self.t)
+            return
         for name, cin, cout, _ in self.layers:
             self.ops.adam(self.W[f"{name}.w"], self.G[f"{name}.w"], self.M[f"{name}.w"], self.V[f"{name}.w"],
                           self.Wb[name], lr, b1, b2, eps, self.t)

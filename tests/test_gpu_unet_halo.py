@@ -164,3 +164,30 @@ def test_masked_loss_forms(gpu, cpad, ct):
     ref[:, :ct] = 2 * cw * d / count
     assert abs(float(loss) - 1 - (cw * d * d).sum() / count) <= 1e-12 * vox
     assert rel_l2(dout.float().cpu().numpy(), ref) <= 2.0 ** -8
+
+
+@pytest.mark.parametrize("replaced", [None, "W", "G"])
+def test_optimiser_on_the_flat_buffers(gpu, replaced):
+    """One launch over the flat buffers and one per tensor (taken when a tensor was replaced by the
+    caller): the same bits."""
+    import torch
+
+    nets = [N.UNet3D(16, seed=3) for _ in range(2)]
+    key = "d2b.w"
+    if replaced:
+        getattr(nets[0], replaced)[key] = getattr(nets[0], replaced)[key].clone()
+    else:  # the per-tensor form as the reference
+        nets[1].M[key] = nets[1].M[key].clone()
+    for step in range(3):
+        for net in nets:
+            net.zero_grad()
+            assert all(float(g.abs().max()) == 0 for g in net.G.values())
+            gen = torch.Generator(device="cuda").manual_seed(step)
+            for k in sorted(net.G):
+                net.G[k].copy_(torch.randn(net.G[k].shape, device="cuda", generator=gen))
+            net.adam_step(lr=1e-2)
+    for k in nets[0].W:
+        assert torch.equal(nets[0].W[k], nets[1].W[k])
+    for k in nets[0].Wb:
+        assert torch.equal(nets[0].Wb[k], nets[1].Wb[k])
+        assert torch.equal(nets[0].Wb[k], nets[0].W[k + ".w"].bfloat16())
