@@ -33,6 +33,14 @@ const char* nn_last_error(void);
 /* out = act(conv3x3x3(in, w) + bias); act = ReLU when relu != 0.  bias may be NULL. */
 int32_t nn_conv3d_fwd(const void* in, const void* w, const float* bias, void* out, int32_t n, int32_t d,
                       int32_t h, int32_t wd, int32_t cin, int32_t cout, int32_t relu, void* stream);
+/* out = act(conv3x3x3([up2(low), skip], w) + bias): the convolution of what nn_up2_concat would
+ * write (cu channels of the coarse grid upsampled, then cs channels of the fine one; fine grid
+ * d, h, wd), without writing it; the same values as the two calls.  Cout 16 or 32, 16-byte
+ * aligned tensors, engines 1 and 2; returns -1 (no error) and does nothing where it does not
+ * apply. */
+int32_t nn_conv3d_up2cat_fwd(const void* low, const void* skip, const void* w, const float* bias, void* out, int32_t n,
+                             int32_t d, int32_t h, int32_t wd, int32_t cu, int32_t cs, int32_t cout, int32_t relu,
+                             void* stream);
 /* Engine of nn_conv3d_fwd (and so of the data gradient): 0 = mma.sync warp tiles
  * (FP32 accumulation in registers); 1 and 2 (default) = tcgen05 on tiles staged in shared
  * memory with their halo, FP32 accumulators in tensor memory (tensors that are not 16-byte

@@ -273,6 +273,11 @@ struct HaloArgs {
   long long sp, sr, sn;          // strides in voxels
   int tap_p, tap_r;              // strides of P and R in the tap index (3 or 9)
   int cin, kcs;                  // input channels and 16-channel slices
+  // concatenated input (UP): the first kcu slices are `low`, nearest-upsampled by two, the rest
+  // the skip tensor; nothing of it is written to memory
+  const bf16* low;
+  int kcu, cu, cs;               // slices and channels of low, channels of the skip tensor
+  long long lp, lr, ln;          // strides of low in voxels
   int br;                        // output planes of a tile along R
   int tx, tp, tr;                // tiles per axis
   int tiles;
@@ -303,7 +308,7 @@ __device__ __forceinline__ void halo_load_weights(uint32_t dst, const bf16* __re
   }
 }
 
-template <int BX>
+template <int BX, bool UP>
 __device__ __forceinline__ void halo_load_slab(uint32_t dst, const bf16* __restrict__ in, const HaloArgs& a, int tile,
                                                int kc, int tid) {
   constexpr int PX = BX + 2, PP = HT_P + 2;
@@ -326,15 +331,37 @@ __device__ __forceinline__ void halo_load_slab(uint32_t dst, const bf16* __restr
     p -= PP;
     r++;
   }
-  const bf16* base = in + (long long)n * a.sn * a.cin + kc * 16 + half * 8;
+  dst += half * a.plane + v * 16;
+  if (UP && kc < a.kcu) {  // eight fine voxels read one coarse voxel
+    const bf16* low = a.low + (long long)n * a.ln * a.cu + kc * 16 + half * 8;
+#pragma unroll 2
+    for (const int end = (a.br + 2) * PP * PX; v < end; v += STEP) {
+      const int gx = x0 + x, gp = p0 + p, gr = r0 + r;
+      const bool ok = (unsigned)gx < (unsigned)a.w && (unsigned)gp < (unsigned)a.np && (unsigned)gr < (unsigned)a.nr;
+      cp_async16(dst, low + (ok ? ((gr >> 1) * a.lr + (gp >> 1) * a.lp + (gx >> 1)) * a.cu : 0), ok);
+      dst += STEP * 16;
+      x += DX;
+      p += DP;
+      if (x >= PX) {
+        x -= PX;
+        p++;
+      }
+      if (p >= PP) {
+        p -= PP;
+        r++;
+      }
+    }
+    return;
+  }
+  const int ci = UP ? a.cs : a.cin, ch = (UP ? kc - a.kcu : kc) * 16 + half * 8;
+  const bf16* base = in + (long long)n * a.sn * ci + ch;
   long long off = (r0 + r) * a.sr + (p0 + p) * a.sp + x0 + x;
   const long long step = DX + DP * a.sp, carry_x = a.sp - PX, carry_p = a.sr - PP * a.sp;
-  dst += half * a.plane + v * 16;
 #pragma unroll 2
   for (const int end = (a.br + 2) * PP * PX; v < end; v += STEP) {
     const bool ok = (unsigned)(x0 + x) < (unsigned)a.w && (unsigned)(p0 + p) < (unsigned)a.np &&
                     (unsigned)(r0 + r) < (unsigned)a.nr;
-    cp_async16(dst, base + (ok ? off * a.cin : 0), ok);
+    cp_async16(dst, base + (ok ? off * ci : 0), ok);
     dst += STEP * 16;
     off += step;
     x += DX;
@@ -352,7 +379,7 @@ __device__ __forceinline__ void halo_load_slab(uint32_t dst, const bf16* __restr
   }
 }
 
-template <int COUT, int BX>
+template <int COUT, int BX, bool UP>
 __global__ void __launch_bounds__(HT_THREADS, 1)
     conv_halo_kernel(const bf16* __restrict__ in, const bf16* __restrict__ w, const float* __restrict__ bias,
                      bf16* __restrict__ out, const HaloArgs a, int* err) {
@@ -389,7 +416,7 @@ __global__ void __launch_bounds__(HT_THREADS, 1)
       for (int k = 0; k < a.kcs; k++) halo_load_weights<COUT>(wbase + k * WSLICE, w, a, k, tid);
     else
       halo_load_weights<COUT>(s0 + a.slab, w, a, 0, tid);
-    halo_load_slab<BX>(s0, in, a, first, 0, tid);
+    halo_load_slab<BX, UP>(s0, in, a, first, 0, tid);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -493,7 +520,7 @@ __global__ void __launch_bounds__(HT_THREADS, 1)
         const int nk = kc + 1 == a.kcs ? 0 : kc + 1, ns = nk ? seq : seq + 1;
         const uint32_t next = s0 + ((it + 1) & 1) * a.stage;
         if (!a.wres) halo_load_weights<COUT>(next + a.slab, w, a, nk, tid);
-        halo_load_slab<BX>(next, in, a, first + ns * stride, nk, tid);
+        halo_load_slab<BX, UP>(next, in, a, first + ns * stride, nk, tid);
       }
       if (ok && kc == 0 && seq > 0) epilogue(seq - 1);
     }
@@ -1598,23 +1625,37 @@ bool halo_plan(const Geo& g, int cin, int cout, int sms, HaloPlan& best) {
   return best_cost < 1e300;
 }
 
-template <int COUT, int BX>
+template <int COUT, int BX, bool UP>
 int halo_launch(const bf16* in, const bf16* w, const float* bias, bf16* out, const HaloPlan& p, int* err,
                 cudaStream_t s) {
   static std::atomic<unsigned long long> done{0};
-  if (!allow_smem(conv_halo_kernel<COUT, BX>, HT_MAX_SMEM, done)) return launched("nn_conv3d_fwd (shared memory)");
-  launch_chained_smem(conv_halo_kernel<COUT, BX>, p.grid, HT_THREADS, p.smem, s, in, w, bias, out, p.a, err);
+  if (!allow_smem(conv_halo_kernel<COUT, BX, UP>, HT_MAX_SMEM, done)) return launched("nn_conv3d_fwd (shared memory)");
+  launch_chained_smem(conv_halo_kernel<COUT, BX, UP>, p.grid, HT_THREADS, p.smem, s, in, w, bias, out, p.a, err);
   return launched("nn_conv3d_fwd (tcgen05)");
 }
 
+// Convolution of `in`, or, with cu > 0, of the nearest-upsampled `low` (cu channels) beside it.
 template <int COUT>
 int halo_conv(const bf16* in, const bf16* w, const float* bias, bf16* out, const Geo& g, int cin, int relu, int* err,
-              cudaStream_t s) {
+              cudaStream_t s, const bf16* low = nullptr, int cu = 0) {
   HaloPlan p{};
-  if (!halo_plan(g, cin, COUT, sm_count(), p)) return fail("nn_conv3d_fwd: no tile for %d x %d x %d", g.d, g.h, g.w);
+  if (!halo_plan(g, cin + cu, COUT, sm_count(), p)) return fail("nn_conv3d_fwd: no tile for %d x %d x %d", g.d, g.h, g.w);
   p.a.relu = relu;
-  return p.bx == 16 ? halo_launch<COUT, 16>(in, w, bias, out, p, err, s)
-                    : halo_launch<COUT, 8>(in, w, bias, out, p, err, s);
+  if (cu) {
+    const bool z_is_p = p.a.tap_p == 9;
+    const long long ly = g.w / 2, lz = ly * (g.h / 2);
+    p.a.low = low;
+    p.a.kcu = cu / 16;
+    p.a.cu = cu;
+    p.a.cs = cin;
+    p.a.lp = z_is_p ? lz : ly;
+    p.a.lr = z_is_p ? ly : lz;
+    p.a.ln = lz * (g.d / 2);
+    return p.bx == 16 ? halo_launch<COUT, 16, true>(in, w, bias, out, p, err, s)
+                      : halo_launch<COUT, 8, true>(in, w, bias, out, p, err, s);
+  }
+  return p.bx == 16 ? halo_launch<COUT, 16, false>(in, w, bias, out, p, err, s)
+                    : halo_launch<COUT, 8, false>(in, w, bias, out, p, err, s);
 }
 
 // Tensor map over channels-last activations seen as (8 channels, x, ...): the 8-channel groups
@@ -1793,6 +1834,22 @@ int32_t nn_conv3d_fwd(const void* in, const void* w, const float* bias, void* ou
     default: return fail("nn_conv3d_fwd: Cout %d not in {16, 32, 48, 64, 96}", cout);
   }
   return launched("nn_conv3d_fwd");
+}
+
+int32_t nn_conv3d_up2cat_fwd(const void* low, const void* skip, const void* w, const float* bias, void* out, int32_t n,
+                             int32_t d, int32_t h, int32_t wd, int32_t cu, int32_t cs, int32_t cout, int32_t relu,
+                             void* stream) {
+  if (!low || !skip || !w || !out || !geo_ok(n, d, h, wd)) return fail("nn_conv3d_up2cat_fwd: null pointer or empty shape");
+  if (wd % 16 || d % 2 || h % 2 || cu % 16 || cs % 16 || cu <= 0 || cs <= 0)
+    return fail("nn_conv3d_up2cat_fwd: W and the channels must be multiples of 16, D and H even");
+  if ((g_engine != 1 && g_engine != 2) || (cout != 16 && cout != 32) || !aligned16(low) || !aligned16(skip) ||
+      !aligned16(w) || !aligned16(out))
+    return -1;
+  int* err = tc_err_ptr();
+  if (!err) return fail("nn_conv3d_up2cat_fwd: no device address for the error word");
+  const auto run = cout == 16 ? halo_conv<16> : halo_conv<32>;
+  return run((const bf16*)skip, (const bf16*)w, bias, (bf16*)out, Geo{n, d, h, wd}, cs, relu, err, (cudaStream_t)stream,
+             (const bf16*)low, cu);
 }
 
 int32_t nn_set_conv_engine(int32_t engine) {

@@ -44,6 +44,7 @@ def lib() -> C.CDLL:
         "nn_abi_version": (i32, []),
         "nn_last_error": (C.c_char_p, []),
         "nn_conv3d_fwd": (i32, [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp]),
+        "nn_conv3d_up2cat_fwd": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp]),
         "nn_conv3d_flip": (i32, [vp, vp, i32, i32, vp]),
         "nn_conv3d_bwd_weight": (i32, [vp, vp, vp, i32, i32, i32, i32, i32, i32, vp]),
         "nn_bias_grad": (i32, [vp, vp, i64, i32, vp]),
@@ -73,7 +74,8 @@ def lib() -> C.CDLL:
 
 
 def exported_symbols() -> list[str]:
-    return ["nn_abi_version", "nn_last_error", "nn_set_conv_engine", "nn_conv_uses_tma", "nn_tc_status", "nn_wait_selftest", "nn_conv3d_fwd", "nn_conv3d_flip", "nn_conv3d_bwd_weight",
+    return ["nn_abi_version", "nn_last_error", "nn_set_conv_engine", "nn_conv_uses_tma", "nn_tc_status", "nn_wait_selftest", "nn_conv3d_fwd",
+            "nn_conv3d_up2cat_fwd", "nn_conv3d_flip", "nn_conv3d_bwd_weight",
             "nn_bias_grad", "nn_relu_bwd", "nn_pool2", "nn_pool2_bwd", "nn_up2_concat", "nn_up2_concat_bwd",
             "nn_mse", "nn_adam", "nn_diff_norms", "nn_features_ellipsoid", "nn_unpack_fields", "nn_to_bf16",
             "nn_from_bf16"]
@@ -115,6 +117,15 @@ class Ops:
     def conv(self, x, w, b, y, shape, cin, cout, relu):
         n, d, h, wd = shape
         _ck(self.L.nn_conv3d_fwd(_p(x), _p(w), _p(b), _p(y), n, d, h, wd, cin, cout, int(relu), self.s))
+
+    def conv_up_cat(self, low, skip, w, b, y, shape, cu, cs, cout, relu) -> bool:
+        """up_cat and conv without the concatenated tensor; False (and nothing done) where the
+        current engine has no such kernel."""
+        n, d, h, wd = shape
+        rc = self.L.nn_conv3d_up2cat_fwd(_p(low), _p(skip), _p(w), _p(b), _p(y), n, d, h, wd, cu, cs, cout, int(relu), self.s)
+        if rc != -1:
+            _ck(rc)
+        return rc == 0
 
     def flip(self, w, wt, cin, cout):
         _ck(self.L.nn_conv3d_flip(_p(w), _p(wt), cin, cout, self.s))
@@ -232,6 +243,9 @@ class UNet3D:
             self.ops.to_bf16(self.W[f"{name}.w"], self.Wb[name])
         self._views = {(n, k): t.data_ptr() for n, d in self._named() for k, t in d.items()}
         self.t = 0
+        w = width
+        self._cat = {"d2a": (4 * w, 2 * w, 2 * w, True), "d1a": (2 * w, w, w, True)}  # cu, cs, cout, relu
+        self._missing = {}  # concatenated activations that the last forward pass left out
         self._shape = None
 
     def _named(self):
@@ -264,6 +278,23 @@ class UNet3D:
         cin, cout, relu = next((ci, co, r) for nm, ci, co, r in self.layers if nm == name)
         self.ops.conv(x, self.Wb[name], self.W[f"{name}.b"], y, self.geo[lv], cin, cout, relu)
 
+    def _conv_up_cat(self, name, low, skip, cat, y, lv):
+        """Convolution of the upsampled and concatenated input; `cat` itself is only written where
+        the engine needs it (backward writes it for the weight gradient)."""
+        A, (cu, cs, cout, relu) = self.A, self._cat[name]
+        done = self.ops.conv_up_cat(A[low], A[skip], self.Wb[name], self.W[f"{name}.b"], A[y], self.geo[lv], cu, cs, cout, relu)
+        if not done:
+            self.ops.up_cat(A[low], A[skip], A[cat], self.geo[lv], cu, cs)
+            self._conv(name, A[cat], A[y], lv)
+        self._missing[cat] = (low, skip, cu, cs, lv) if done else None
+
+    def _concatenated(self, cat):
+        if self._missing.get(cat):
+            low, skip, cu, cs, lv = self._missing[cat]
+            self.ops.up_cat(self.A[low], self.A[skip], self.A[cat], self.geo[lv], cu, cs)
+            self._missing[cat] = None
+        return self.A[cat]
+
     def forward(self, x):
         """x: BF16 (n, d, h, w, 16) with w % 64 == 0 and d, h % 4 == 0; returns the
         BF16 output buffer (n, d, h, w, 16), valid until the next call."""
@@ -279,11 +310,9 @@ class UNet3D:
         o.pool(A["s2"], A["p2"], self.geo[2], 2 * w)
         self._conv("e3a", A["p2"], A["a3"], 3)
         self._conv("e3b", A["a3"], A["b3"], 3)
-        o.up_cat(A["b3"], A["s2"], A["c2"], self.geo[2], 4 * w, 2 * w)
-        self._conv("d2a", A["c2"], A["a4"], 2)
+        self._conv_up_cat("d2a", "b3", "s2", "c2", "a4", 2)
         self._conv("d2b", A["a4"], A["a5"], 2)
-        o.up_cat(A["a5"], A["s1"], A["c1"], self.geo[1], 2 * w, w)
-        self._conv("d1a", A["c1"], A["a6"], 1)
+        self._conv_up_cat("d1a", "a5", "s1", "c1", "a6", 1)
         self._conv("d1b", A["a6"], A["a7"], 1)
         self._conv("head", A["a7"], A["out"], 1)
         return A["out"]
@@ -309,10 +338,10 @@ class UNet3D:
         D["out"].copy_(dout) if dout.data_ptr() != D["out"].data_ptr() else None
         self._back("head", A["a7"], D["out"], D["a7"], 1)
         self._back("d1b", A["a6"], D["a7"], D["a6"], 1, A["a7"])
-        self._back("d1a", A["c1"], D["a6"], D["c1"], 1, A["a6"])
+        self._back("d1a", self._concatenated("c1"), D["a6"], D["c1"], 1, A["a6"])
         o.up_cat_bwd(D["c1"], D["a5"], D["s1"], self.geo[1], 2 * w, w)
         self._back("d2b", A["a4"], D["a5"], D["a4"], 2, A["a5"])
-        self._back("d2a", A["c2"], D["a4"], D["c2"], 2, A["a4"])
+        self._back("d2a", self._concatenated("c2"), D["a4"], D["c2"], 2, A["a4"])
         o.up_cat_bwd(D["c2"], D["b3"], D["s2"], self.geo[2], 4 * w, 2 * w)
         self._back("e3b", A["a3"], D["b3"], D["a3"], 3, A["b3"])
         self._back("e3a", A["p2"], D["a3"], D["p2"], 3, A["a3"])

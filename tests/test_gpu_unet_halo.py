@@ -191,3 +191,28 @@ def test_optimiser_on_the_flat_buffers(gpu, replaced):
     for k in nets[0].Wb:
         assert torch.equal(nets[0].Wb[k], nets[1].Wb[k])
         assert torch.equal(nets[0].Wb[k], nets[0].W[k + ".w"].bfloat16())
+
+
+@pytest.mark.parametrize("shape,cu,cs,cout", [((1, 2, 2, 16), 32, 16, 16), ((2, 6, 18, 32), 64, 32, 32),
+                                              ((1, 34, 4, 16), 32, 16, 32), ((2, 20, 34, 64), 32, 16, 16)])
+def test_convolution_of_an_upsampled_concatenation(gpu, shape, cu, cs, cout):
+    """The same bits as nn_up2_concat followed by nn_conv3d_fwd; refused by the other engines."""
+    import torch
+
+    ops = N.Ops()
+    rng = np.random.default_rng(sum(shape) + cu)
+    n, d, h, w = shape
+    low, skip = (_bf16(rng.standard_normal(s)) for s in ((n, d // 2, h // 2, w // 2, cu), shape + (cs,)))
+    wt, b = _bf16(rng.standard_normal((27, cout, cu + cs)) / 20), torch.from_numpy(rng.standard_normal(cout).astype(np.float32)).cuda()
+    cat, y0, y1 = (torch.empty(shape + (c,), dtype=torch.bfloat16, device="cuda") for c in (cu + cs, cout, cout))
+    ops.up_cat(low, skip, cat, shape, cu, cs)
+    ops.conv(cat, wt, b, y0, shape, cu + cs, cout, True)
+    assert ops.conv_up_cat(low, skip, wt, b, y1, shape, cu, cs, cout, True)
+    N.tc_status()
+    assert torch.equal(y0, y1)
+    for engine in ("mma", "tcgen05-tma"):
+        prev = N.set_conv_engine(engine)
+        try:
+            assert not ops.conv_up_cat(low, skip, wt, b, y1, shape, cu, cs, cout, True)
+        finally:
+            N.set_conv_engine(prev)
