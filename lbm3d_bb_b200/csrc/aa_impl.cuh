@@ -40,11 +40,16 @@
 #define LBM_MINB_F16 4
 #endif
 
-// blocks of BATCH_ITEM threads per SM that the batched kernel's register budget allows:
-// FP32 6 (80 registers; 2 % faster than 8 on the 512-domain sweep, 4 was slower), the
-// other storages 2 x MIN_BLOCKS
+// Blocks of BATCH_ITEM threads per SM that the batched kernel's register budget allows:
+// five in FP32 and FP16-deviation (96 registers), three in FP64 (168).  The kernel waits
+// for its loads, which a thread issues together only while it has registers to hold them,
+// so fewer warps with more loads in flight each win until too few warps are left.
+// Measured on B200, us per step of 8 / 16 / 64 body-fitted domains (BGK, x force):
+//   FP32   4: 38.9/93.9/430   5: 38.6/87.8/394   6: 42.5/92.7/401   7: 44.9/94.8/412
+//   FP16   5: 47.1/91.2/407   6: 48.5/98.7/407   8: 52.7/104/425
+//   FP64   3: 58.9/136/629    4: 66.2/143/645    5: 77.4/161/720
 #ifndef LBM_BATCH_MINB
-#define LBM_BATCH_MINB(SP) (sizeof(typename SP::S) == 4 ? 6 : 2 * SP::MIN_BLOCKS)
+#define LBM_BATCH_MINB(SP) (sizeof(typename SP::S) == 8 ? 3 : 5)
 #endif
 
 namespace lbm {
