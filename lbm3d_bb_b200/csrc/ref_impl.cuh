@@ -272,8 +272,16 @@ __device__ __forceinline__ void ref_pull(const RefParams& p, const T* __restrict
   }
 }
 
+// Blocks of 256 threads per SM that the register budget of the step is made for.  FP32 D3Q19:
+// three (80 registers); left alone the compiler takes 64, spills 60 bytes and holds back
+// loads.  B200, us per step, left alone / two / three / five blocks: 480x240x4 23.0 / 22.3 /
+// 22.2 / 25.0, 700x480x12 155 / 148 / 141.5 / 168.  FP32 D3Q27 is best left alone (203 / 211 /
+// 213 / 266 at 700x480x12), and FP64 needs more registers than three blocks leave.
+template <class T>
+constexpr int REF_MIN_BLOCKS = sizeof(T) == 4 && Q == 19 ? 3 : 0;
+
 template <class T, bool TRT>
-__global__ void __launch_bounds__(256) ref_step_kernel(const __grid_constant__ RefParams p,
+__global__ void __launch_bounds__(256, REF_MIN_BLOCKS<T>) ref_step_kernel(const __grid_constant__ RefParams p,
                                                        const T* __restrict__ Fp, const T* __restrict__ Rp,
                                                        T* __restrict__ Fn, T* __restrict__ Rn,
                                                        const uint8_t* __restrict__ flags) {
