@@ -79,7 +79,8 @@ def step_kernel(storage: str, n: int) -> str:
         return "aa_step_kernel"
     if storage == "fp16dev":
         quad = os.environ.get("LBM3D_QUAD") != "0"
-        octo = quad and n % 256 == 0 and os.environ.get("LBM3D_OCTO") != "0"
+        octo_env = os.environ.get("LBM3D_OCTO")
+        octo = quad and n % 256 == 0 and (octo_env != "0" if octo_env else n ** 3 >= 64 << 20)
         even = "aa_octo_even_kernel" if octo else ("aa_quad_even_kernel" if quad else "aa_pair_kernel")
         return even + " / aa_pair_split_kernel"
     return "aa_pair_kernel"

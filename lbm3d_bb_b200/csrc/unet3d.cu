@@ -1854,7 +1854,7 @@ int32_t nn_conv3d_up2cat_fwd(const void* low, const void* skip, const void* w, c
 
 int32_t nn_set_conv_engine(int32_t engine) {
   if (engine < 0 || engine > 3) {
-    fail("nn_set_conv_engine: engine must be 0 (mma.sync), 1 (tcgen05), 2 (per layer) or 3 (tcgen05, TMA-fed)");
+    fail("nn_set_conv_engine: engine must be 0 (mma.sync), 1 (tcgen05), 2 (the default, tcgen05 as well) or 3 (tcgen05, TMA-fed)");
     return -1;
   }
   const int prev = g_engine;
