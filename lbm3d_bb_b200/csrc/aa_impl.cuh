@@ -828,8 +828,12 @@ __device__ __forceinline__ void aa_direct(const AAParams& p, typename SP::S* __r
   }
 }
 
+// The moving-link instantiation keeps the node's populations across a call per link, so three
+// blocks (80 registers) serve it better than four: us per step with poses, B200, 4 / 3 blocks,
+// FP32 192x96x96 BGK 73.0 / 69.7, TRT 75.5 / 70.8, 96x64x64 33.2 / 32.7, FP16 192x96x96
+// 62.4 / 59.6.  The other instantiations lose with three (FP32 channel 331x160x160 262 / 274).
 template <class SP, bool ODD, bool TRT, int FORCE, bool FACES, bool MOVE>
-__global__ void __launch_bounds__(256, SP::MIN_BLOCKS) aa_step_kernel(const __grid_constant__ AAParams p,
+__global__ void __launch_bounds__(256, MOVE && SP::MIN_BLOCKS > 3 ? 3 : SP::MIN_BLOCKS) aa_step_kernel(const __grid_constant__ AAParams p,
                                                                       typename SP::S* __restrict__ A,
                                                                       const uint8_t* __restrict__ flags) {
   const Grid& g = p.g;
