@@ -1085,8 +1085,8 @@ int32_t lbm_step(lbm_ctx* c, int32_t nsteps) {
       p.zero_next = next;
       // a moving body in a box with faces: one cell per thread, links on the fast path
       // up to 6 M cells, 2 M for BGK in FP16 deviations (B200, us per step, other rule / this:
-      // FP32 TRT 192x96x96 87 / 79, BGK 240x150x140 182 / 174, 384x205x199 466 / 478; FP16
-      // TRT 192x96x96 75 / 67, BGK 240x150x140 159 / 163)
+      // FP32 TRT 192x96x96 87 / 72, BGK 280x150x150 218 / 216, 331x160x160 289 / 298; FP16
+      // TRT 192x96x96 75 / 63, 331x160x160 273 / 281, BGK 256x128x128 130 / 146)
       const bool bgk16 = c->cfg.storage == LBM_STORE_FP16DEV && !trt;
       p.move = c->has_moving && has_faces(c) && c->g.N < (bgk16 ? 2000000 : 6000000);
       p.pair = c->pair ? 1 : (c->rows && !p.move ? 2 : 0);
