@@ -387,14 +387,14 @@ __global__ void __launch_bounds__(FT_X* FT_Y* FT_Z) body_flags_kernel(const __gr
   constexpr int HX = FT_X + 2, HY = FT_Y + 2, HZ = FT_Z + 2;
   __shared__ uint8_t tile[HZ][HY][HX];  // 0 outside the box of nodes
   const int n3[3] = {g.nx, g.ny, g.nz};
-  const bool wrap = p.mode == LBM_MODE_CONFIG;
   const int o[3] = {rn.lo[0] + (int)blockIdx.x * FT_X, rn.lo[1] + (int)blockIdx.y * FT_Y,
                     rn.lo[2] + (int)blockIdx.z * FT_Z};
   const int tid = threadIdx.x + FT_X * (threadIdx.y + FT_Y * threadIdx.z);
-  // a node beyond a non-periodic end (every end in reference mode) is no neighbour
+  // which node a coordinate of the box is: boxes run across the ends of a periodic axis in both
+  // modes (z in reference mode); beyond other ends there is none
   const auto node = [&](int a, int c) -> int {
     if (c >= 0 && c < n3[a]) return c;
-    return wrap && g.per[a] ? wrap1(c, n3[a]) : -1;
+    return g.per[a] ? wrap1(c, n3[a]) : -1;
   };
   for (int k = tid; k < HX * HY * HZ; k += FT_X * FT_Y * FT_Z) {
     const int hx = k % HX, hy = k / HX % HY, hz = k / (HX * HY);
@@ -422,10 +422,14 @@ __global__ void __launch_bounds__(FT_X* FT_Y* FT_Z) body_flags_kernel(const __gr
   const int tx = threadIdx.x + 1, ty = threadIdx.y + 1, tz = threadIdx.z + 1;
   const uint8_t fl = tile[tz][ty][tx];
   const bool sc = fl & F_SOLID, sp = fl & F_SOLID_PREV;
+  // reference mode: the nodes on the two sides of the z wrap are not neighbours
+  const bool config = p.mode == LBM_MODE_CONFIG;
+  const bool zlo = !config && z == 0, zhi = !config && z == g.nz - 1;
   bool near = sp && !sc;
   unsigned long long lw = 0;
 #pragma unroll
   for (int d = 0; d < 18; d++) {
+    if ((cz(d) > 0 && zlo) || (cz(d) < 0 && zhi)) continue;
     const uint8_t fn = tile[tz - cz(d)][ty - cy(d)][tx - cx(d)];
     if (fn & (F_SOLID | F_SOLID_PREV)) near = true;
     if (fn & F_SOLID) lw |= 1ull << d;
@@ -433,8 +437,10 @@ __global__ void __launch_bounds__(FT_X* FT_Y* FT_Z) body_flags_kernel(const __gr
     if (fn & F_MOVING) lw |= 1ull << (36 + d);
   }
   if (g.q == 27)
-    for (int d = 18; d < 26; d++)
+    for (int d = 18; d < 26; d++) {
+      if ((cz27(d) > 0 && zlo) || (cz27(d) < 0 && zhi)) continue;
       if (tile[tz - cz27(d)][ty - cy27(d)][tx - cx27(d)] & (F_SOLID | F_SOLID_PREV)) near = true;
+    }
   near = near && (!sc || !sp);
   flags[i] = near ? (uint8_t)(fl | F_NEAR) : fl;
   if (links) links[i] = lw;
