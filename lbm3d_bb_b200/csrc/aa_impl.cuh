@@ -776,7 +776,8 @@ __device__ __forceinline__ bool ghost_plane(const AAParams& p, const int z) {
 // neighbour offsets wrap).  Without FACES (all axes periodic) the same rule holds;
 // with FACES, nodes on non-periodic faces are fast too (face mask).
 // MOVE: links to a moving body stay on the fast path as long as the node's solid neighbours are
-// those of the last step.
+// those of the last step.  A node that also lies on a face does not: its link values replace
+// outgoing populations that face values are made of (an outflow face stores pst[d] itself).
 template <class SP, bool ODD, bool TRT, int FORCE, bool FACES, bool MOVE = false>
 __device__ __forceinline__ void aa_direct(const AAParams& p, typename SP::S* __restrict__ A,
                                           const uint8_t* __restrict__ flags, const int x, const int y, const int z,
@@ -815,7 +816,7 @@ __device__ __forceinline__ void aa_direct(const AAParams& p, typename SP::S* __r
     const unsigned long long lw = p.links[i];
     const uint32_t cur = (uint32_t)(lw & 0x3FFFFu), prev = (uint32_t)((lw >> 18) & 0x3FFFFu);
     const uint32_t mov = (uint32_t)((lw >> 36) & 0x3FFFFu);
-    static_links = cur == prev && (MOVE || mov == 0) && !(fl & F_SOLID_PREV);
+    static_links = cur == prev && (mov == 0 || (MOVE && fc.mask == 0)) && !(fl & F_SOLID_PREV);
     bc = cur;
     if (MOVE) moving = mov & cur;
   }
