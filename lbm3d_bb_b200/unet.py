@@ -210,6 +210,41 @@ def init_params(width: int = 16, seed: int = 0, n_inputs: int = 6) -> dict[str, 
     return params
 
 
+class _Activations(dict):
+    """Activation buffers by name.  Those named in `sources` were left out by a forward pass (the
+    convolution reads its two sources in place); they are written whenever they are asked for, and
+    every time, because their sources may be newer (a forward pass replayed from a graph runs no
+    Python)."""
+
+    def __init__(self, ops, buffers):
+        super().__init__(buffers)
+        self.ops = ops
+        self.sources = {}
+
+    def __getitem__(self, name):
+        out = super().__getitem__(name)
+        if name in self.sources:
+            low, skip, geo, cu, cs = self.sources[name]
+            self.ops.up_cat(self[low], self[skip], out, geo, cu, cs)
+        return out
+
+    def __iter__(self):  # its own, so that dict(activations) asks for every item
+        return super().__iter__()
+
+    def buffers(self) -> dict:
+        """The buffers as they are, in a plain dict."""
+        return {name: dict.__getitem__(self, name) for name in dict.keys(self)}
+
+    def get(self, name, default=None):
+        return self[name] if name in self else default
+
+    def items(self):
+        return [(name, self[name]) for name in self]
+
+    def values(self):
+        return [self[name] for name in self]
+
+
 class UNet3D:
     """Parameters on one GPU plus the forward / backward passes for a batch shape."""
 
@@ -245,7 +280,6 @@ class UNet3D:
         self.t = 0
         w = width
         self._cat = {"d2a": (4 * w, 2 * w, 2 * w, True), "d1a": (2 * w, w, w, True)}  # cu, cs, cout, relu
-        self._missing = {}  # concatenated activations that the last forward pass left out
         self._shape = None
 
     def _named(self):
@@ -268,7 +302,7 @@ class UNet3D:
                  "p2": (3, 2 * w), "a3": (3, 4 * w), "b3": (3, 4 * w), "c2": (2, 6 * w), "a4": (2, 2 * w),
                  "a5": (2, 2 * w), "c1": (1, 3 * w), "a6": (1, w), "a7": (1, w), "out": (1, OUT_CH)}
         bf = dict(dtype=t.bfloat16, device=self.dev)
-        self.A = {k: t.empty((*self.geo[lv], c), **bf) for k, (lv, c) in chans.items()}
+        self.A = _Activations(self.ops, {k: t.empty((*self.geo[lv], c), **bf) for k, (lv, c) in chans.items()})
         self.D = {k: t.empty((*self.geo[lv], c), **bf) for k, (lv, c) in chans.items() if k != "x"}
         self.Wt = {name: t.empty((27, cin, cout), **bf) for name, cin, cout, _ in self.layers}
         self._shape = shape
@@ -278,29 +312,22 @@ class UNet3D:
         cin, cout, relu = next((ci, co, r) for nm, ci, co, r in self.layers if nm == name)
         self.ops.conv(x, self.Wb[name], self.W[f"{name}.b"], y, self.geo[lv], cin, cout, relu)
 
-    def _conv_up_cat(self, name, low, skip, cat, y, lv):
-        """Convolution of the upsampled and concatenated input; `cat` itself is only written where
-        the engine needs it (backward writes it for the weight gradient)."""
-        A, (cu, cs, cout, relu) = self.A, self._cat[name]
-        done = self.ops.conv_up_cat(A[low], A[skip], self.Wb[name], self.W[f"{name}.b"], A[y], self.geo[lv], cu, cs, cout, relu)
-        if not done:
-            self.ops.up_cat(A[low], A[skip], A[cat], self.geo[lv], cu, cs)
-            self._conv(name, A[cat], A[y], lv)
-        self._missing[cat] = (low, skip, cu, cs, lv) if done else None
-
-    def _concatenated(self, cat):
-        if self._missing.get(cat):
-            low, skip, cu, cs, lv = self._missing[cat]
-            self.ops.up_cat(self.A[low], self.A[skip], self.A[cat], self.geo[lv], cu, cs)
-            self._missing[cat] = None
-        return self.A[cat]
+    def _conv_up_cat(self, A, name, low, skip, cat, y, lv):
+        """Convolution of the upsampled and concatenated input; where the engine reads the two in
+        place, `cat` is written only for who asks for it (backward, for the weight gradient)."""
+        geo, (cu, cs, cout, relu) = self.geo[lv], self._cat[name]
+        if self.ops.conv_up_cat(A[low], A[skip], self.Wb[name], self.W[f"{name}.b"], A[y], geo, cu, cs, cout, relu):
+            self.A.sources[cat] = (low, skip, geo, cu, cs)
+            return
+        self.ops.up_cat(A[low], A[skip], A[cat], geo, cu, cs)
+        self._conv(name, A[cat], A[y], lv)
 
     def forward(self, x):
         """x: BF16 (n, d, h, w, 16) with w % 64 == 0 and d, h % 4 == 0; returns the
         BF16 output buffer (n, d, h, w, 16), valid until the next call."""
         shape = tuple(int(s) for s in x.shape[:4])
         self._alloc(shape)
-        A, o, w = self.A, self.ops, self.width
+        A, o, w = self.A.buffers(), self.ops, self.width
         A["x"].copy_(x)
         self._conv("e1a", A["x"], A["a1"], 1)
         self._conv("e1b", A["a1"], A["s1"], 1)
@@ -310,9 +337,9 @@ class UNet3D:
         o.pool(A["s2"], A["p2"], self.geo[2], 2 * w)
         self._conv("e3a", A["p2"], A["a3"], 3)
         self._conv("e3b", A["a3"], A["b3"], 3)
-        self._conv_up_cat("d2a", "b3", "s2", "c2", "a4", 2)
+        self._conv_up_cat(A, "d2a", "b3", "s2", "c2", "a4", 2)
         self._conv("d2b", A["a4"], A["a5"], 2)
-        self._conv_up_cat("d1a", "a5", "s1", "c1", "a6", 1)
+        self._conv_up_cat(A, "d1a", "a5", "s1", "c1", "a6", 1)
         self._conv("d1b", A["a6"], A["a7"], 1)
         self._conv("head", A["a7"], A["out"], 1)
         return A["out"]
@@ -334,14 +361,14 @@ class UNet3D:
     def backward(self, dout):
         """dout: gradient of the loss at the output (BF16, like forward's result).
         Adds into the FP32 gradients (zero them with zero_grad)."""
-        A, D, o, w = self.A, self.D, self.ops, self.width
+        A, D, o, w = self.A.buffers(), self.D, self.ops, self.width
         D["out"].copy_(dout) if dout.data_ptr() != D["out"].data_ptr() else None
         self._back("head", A["a7"], D["out"], D["a7"], 1)
         self._back("d1b", A["a6"], D["a7"], D["a6"], 1, A["a7"])
-        self._back("d1a", self._concatenated("c1"), D["a6"], D["c1"], 1, A["a6"])
+        self._back("d1a", self.A["c1"], D["a6"], D["c1"], 1, A["a6"])
         o.up_cat_bwd(D["c1"], D["a5"], D["s1"], self.geo[1], 2 * w, w)
         self._back("d2b", A["a4"], D["a5"], D["a4"], 2, A["a5"])
-        self._back("d2a", self._concatenated("c2"), D["a4"], D["c2"], 2, A["a4"])
+        self._back("d2a", self.A["c2"], D["a4"], D["c2"], 2, A["a4"])
         o.up_cat_bwd(D["c2"], D["b3"], D["s2"], self.geo[2], 4 * w, 2 * w)
         self._back("e3b", A["a3"], D["b3"], D["a3"], 3, A["b3"])
         self._back("e3a", A["p2"], D["a3"], D["p2"], 3, A["a3"])
