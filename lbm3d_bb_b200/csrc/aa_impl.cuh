@@ -389,7 +389,7 @@ __device__ __forceinline__ C face_value(const AAParams& p, const int d, const bo
 // occupancy of the interior fast path; only warps containing a boundary node run it.
 template <class SP, bool ODD, bool TRT, int FORCE>
 __device__ __noinline__ void aa_general(const AAParams& p, typename SP::S* __restrict__ A,
-                                        const uint8_t* __restrict__ flags, const int x, const int y,
+                                        const uint8_t* flags, const int x, const int y,
                                         const int z, const long long i, const uint8_t fl, double* acc,
                                         bool* has_out) {
   using C = typename SP::C;
@@ -780,7 +780,7 @@ __device__ __forceinline__ bool ghost_plane(const AAParams& p, const int z) {
 // outgoing populations that face values are made of (an outflow face stores pst[d] itself).
 template <class SP, bool ODD, bool TRT, int FORCE, bool FACES, bool MOVE = false>
 __device__ __forceinline__ void aa_direct(const AAParams& p, typename SP::S* __restrict__ A,
-                                          const uint8_t* __restrict__ flags, const int x, const int y, const int z,
+                                          const uint8_t* flags, const int x, const int y, const int z,
                                           const bool inb, double* acc, bool* has_link) {
   using C = typename SP::C;
   const Grid& g = p.g;
@@ -836,7 +836,7 @@ __device__ __forceinline__ void aa_direct(const AAParams& p, typename SP::S* __r
 template <class SP, bool ODD, bool TRT, int FORCE, bool FACES, bool MOVE>
 __global__ void __launch_bounds__(256, MOVE && SP::MIN_BLOCKS > 3 ? 3 : SP::MIN_BLOCKS) aa_step_kernel(const __grid_constant__ AAParams p,
                                                                       typename SP::S* __restrict__ A,
-                                                                      const uint8_t* __restrict__ flags) {
+                                                                      const uint8_t* flags) {
   const Grid& g = p.g;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
@@ -935,7 +935,7 @@ __device__ __forceinline__ void pair_cell_x(const AAParams& p, const typename SP
 // take the one-cell path for both cells.
 template <class SP, bool ODD, bool TRT, int FORCE, bool FACES = false>
 __device__ __forceinline__ void pair_cells(const AAParams& p, typename SP::S* __restrict__ A,
-                                           const uint8_t* __restrict__ flags, const int x0, const int y, const int z,
+                                           const uint8_t* flags, const int x0, const int y, const int z,
                                            const bool inb, double* acc, bool& has_link) {
   using S = typename SP::S;
   using C = typename SP::C;
@@ -1097,7 +1097,7 @@ constexpr int pair_blocks() {
 template <class SP, bool ODD, bool TRT, int FORCE>
 __global__ void __launch_bounds__(PAIR_X, pair_blocks<SP, TRT>()) aa_pair_kernel(const __grid_constant__ AAParams p,
                                                                                 typename SP::S* __restrict__ A,
-                                                                                const uint8_t* __restrict__ flags) {
+                                                                                const uint8_t* flags) {
   const Grid& g = p.g;
   const int x0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1124,7 +1124,7 @@ constexpr int ROWS_BLOCK = 128;
 template <class SP, bool ODD, bool TRT, int FORCE, bool FACES>
 __global__ void __launch_bounds__(ROWS_BLOCK, TRT ? 5 : 6) aa_rows_kernel(const __grid_constant__ AAParams p,
                                                                                 typename SP::S* __restrict__ A,
-                                                                                const uint8_t* __restrict__ flags) {
+                                                                                const uint8_t* flags) {
   const Grid& g = p.g;
   const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, half = (unsigned)g.nx / 2;
   const int z = blockIdx.y;
@@ -1151,7 +1151,7 @@ __global__ void __launch_bounds__(ROWS_BLOCK, TRT ? 5 : 6) aa_rows_kernel(const 
 template <class SP, bool TRT, int FORCE>
 __global__ void __launch_bounds__(256, (SP::MIN_BLOCKS > 2 ? 3 : 1)) aa_pair_odd_kernel(const __grid_constant__ AAParams p,
                                                                                     typename SP::S* __restrict__ A,
-                                                                                    const uint8_t* __restrict__ flags) {
+                                                                                    const uint8_t* flags) {
   using S = typename SP::S;
   using C = typename SP::C;
   static_assert(sizeof(S) == 4 && !SP::DEV, "FP32 storage");
@@ -1249,7 +1249,7 @@ __global__ void __launch_bounds__(256, (SP::MIN_BLOCKS > 2 ? 3 : 1)) aa_pair_odd
 // lanes of the warp take part (warp vote).
 template <class SP, bool TRT, int FORCE>
 __device__ __forceinline__ void pair_split_cells(const AAParams& p, typename SP::S* __restrict__ A,
-                                                 const uint8_t* __restrict__ flags, const int x0, const int y,
+                                                 const uint8_t* flags, const int x0, const int y,
                                                  const int z, const bool inb, double* acc, bool& has_link) {
   using S = typename SP::S;
   using C = typename SP::C;
@@ -1375,7 +1375,7 @@ __device__ __forceinline__ void pair_split_cells(const AAParams& p, typename SP:
 template <class SP, bool TRT, int FORCE>
 __global__ void __launch_bounds__(PAIR_X * SPLIT_ROWS, 6) aa_pair_split_kernel(const __grid_constant__ AAParams p,
                                                                                 typename SP::S* __restrict__ A,
-                                                                                const uint8_t* __restrict__ flags) {
+                                                                                const uint8_t* flags) {
   const Grid& g = p.g;
   const int x0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1400,7 +1400,7 @@ __global__ void __launch_bounds__(PAIR_X * SPLIT_ROWS, 6) aa_pair_split_kernel(c
 template <bool TRT, int FORCE>
 __global__ void __launch_bounds__(32 * QUAD_ROWS, 8) aa_quad_even_kernel(const __grid_constant__ AAParams p,
                                                               __half* __restrict__ A,
-                                                              const uint8_t* __restrict__ flags) {
+                                                              const uint8_t* flags) {
   using SP = StF16;
   using C = float;
   const Grid& g = p.g;
@@ -1519,7 +1519,7 @@ __device__ __forceinline__ void u4set(uint4& v, const int k, const uint32_t u) {
 template <bool TRT, int FORCE>
 __global__ void __launch_bounds__(32 * OCTO_ROWS, 6) aa_octo_even_kernel(const __grid_constant__ AAParams p,
                                                               __half* __restrict__ A,
-                                                              const uint8_t* __restrict__ flags) {
+                                                              const uint8_t* flags) {
   using SP = StF16;
   using C = float;
   const Grid& g = p.g;
@@ -1628,7 +1628,7 @@ __host__ __device__ constexpr int xslot(int d) {
 // line, which keeps the word path's code compact.
 template <bool TRT, int FORCE>
 __device__ __noinline__ void odd_pairs_fallback(const AAParams& p, __half* __restrict__ A,
-                                                const uint8_t* __restrict__ flags, const int x0, const int pairs,
+                                                const uint8_t* flags, const int x0, const int pairs,
                                                 const int y, const int z, const bool inb, double* acc, bool* has_out) {
   bool has_link = *has_out;
 #pragma unroll 1
@@ -1666,7 +1666,7 @@ __device__ __forceinline__ void st_u2_masked(char* q, const uint2 v, const uint3
 template <bool TRT, int FORCE>
 __global__ void __launch_bounds__(256, 2) aa_quad_odd_kernel(const __grid_constant__ AAParams p,
                                                              __half* __restrict__ A,
-                                                             const uint8_t* __restrict__ flags) {
+                                                             const uint8_t* flags) {
   using SP = StF16;
   using C = float;
   const Grid& g = p.g;

@@ -12,6 +12,9 @@ namespace lbm {
 // 480x240x4 26.8 -> 25.2).  Launched any other way, chain_begin() does nothing.
 // A kernel that allocates tensor memory triggers after its allocation: a block of the next kernel
 // that took the columns first would wait for this kernel, and this one for the columns.
+// What the kernels before it wrote, a chained kernel reads with ordinary loads: it lives from
+// before they end, and the read-only path (__ldg, const pointers declared __restrict__, which
+// the compiler may load that way) is for data that nobody writes while a kernel lives.
 __device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_begin() {

@@ -145,7 +145,7 @@ __device__ __forceinline__ float ibb_phi(const IbbGeom& b, float x, float y) {
 }
 
 template <class T>
-__device__ __forceinline__ T ref_ibb(const RefParams& p, const T* __restrict__ Fp, T rho_w, int x, int y, int z,
+__device__ __forceinline__ T ref_ibb(const RefParams& p, const T* Fp, T rho_w, int x, int y, int z,
                                      long long i, int dir) {
   const Grid& g = p.g;
   const float h = p.h;
@@ -186,8 +186,8 @@ __device__ __forceinline__ T ref_ibb(const RefParams& p, const T* __restrict__ F
 // (Streaming.jl:82-111, OtherBC.jl:65-82, SolidBC.jl:160-210, OtherBC.jl:112-169),
 // accumulating the momentum exchange (MEA.jl:93-113).
 template <class T>
-__device__ __forceinline__ void ref_pull(const RefParams& p, const T* __restrict__ Fp,
-                                         const T* __restrict__ Rp, const uint8_t* __restrict__ flags,
+__device__ __forceinline__ void ref_pull(const RefParams& p, const T* Fp,
+                                         const T* Rp, const uint8_t* flags,
                                          int x, int y, int z, long long i, T* S, double* acc, bool& has) {
   const Grid& g = p.g;
   const long long nxl = g.nx, nxy = (long long)g.nx * g.ny;
@@ -282,9 +282,9 @@ constexpr int REF_MIN_BLOCKS = sizeof(T) == 4 && Q == 19 ? 3 : 0;
 
 template <class T, bool TRT>
 __global__ void __launch_bounds__(256, REF_MIN_BLOCKS<T>) ref_step_kernel(const __grid_constant__ RefParams p,
-                                                       const T* __restrict__ Fp, const T* __restrict__ Rp,
+                                                       const T* Fp, const T* Rp,
                                                        T* __restrict__ Fn, T* __restrict__ Rn,
-                                                       const uint8_t* __restrict__ flags) {
+                                                       const uint8_t* flags) {
   const Grid& g = p.g;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;

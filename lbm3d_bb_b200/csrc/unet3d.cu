@@ -1,14 +1,13 @@
-// unet3d.cu — kernels of the learned warm start (include/unet3d.h): 3x3x3
-// convolutions as implicit GEMMs on the BF16 tensor cores (FP32 accumulation), their data and weight gradients, 2x pooling / upsampling with
-// skip concatenation, the masked MSE loss and Adam.
+// unet3d.cu — kernels of the learned warm start (include/unet3d.h): 3x3x3 convolutions as
+// implicit GEMMs on the BF16 tensor cores (FP32 accumulation), their data and weight gradients,
+// 2x pooling / upsampling with skip concatenation, the masked MSE loss and Adam.
 //
 // Forward (and data-gradient) convolution: halo tiles on tcgen05 (conv_halo_kernel).  The
 // warp tiles (conv_fwd_kernel, mma.sync) take tensors that are not 16-byte aligned and are an
 // engine of their own: one warp computes 16 consecutive voxels along x by all output
 // channels, K runs over the 27 taps and 16-channel slices, A fragments come straight from the
-// channels-last activations, B fragments from the [tap][Cout][Cin] weights, both through the
-// read-only cache.  Taps whose row lies outside the box are skipped warp-uniformly; voxels
-// outside the row read zero.
+// channels-last activations, B fragments from the [tap][Cout][Cin] weights.  Taps whose row lies
+// outside the box are skipped warp-uniformly; voxels outside the row read zero.
 //
 // Weight gradient: dW[tap] = dY^T X_shift is a GEMM whose reduction runs over the voxels:
 // tcgen05 on slabs staged by TMA (conv_bwdw_tc_kernel).  conv_bwdw_kernel takes what a tensor
@@ -85,8 +84,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 
 // ---- forward convolution ------------------------------------------------------------
 template <int NT>  // output channels / 8
-__global__ void __launch_bounds__(128) conv_fwd_kernel(const bf16* __restrict__ in, const bf16* __restrict__ w,
-                                                       const float* __restrict__ bias, bf16* __restrict__ out,
+__global__ void __launch_bounds__(128) conv_fwd_kernel(const bf16* in, const bf16* w,
+                                                       const float* bias, bf16* __restrict__ out,
                                                        const Geo g, const int cin, const int relu,
                                                        const long long tiles) {
   chain_begin();
@@ -125,14 +124,14 @@ __global__ void __launch_bounds__(128) conv_fwd_kernel(const bf16* __restrict__ 
         const uint32_t* wt = w32 + ((long long)tap * COUT + gid) * cw + tig;
         for (int k2 = 0; k2 < cw; k2 += 8) {
           uint32_t a[4];
-          a[0] = va ? __ldg(pa + k2) : 0u;
-          a[1] = vb ? __ldg(pb + k2) : 0u;
-          a[2] = va ? __ldg(pa + k2 + 4) : 0u;
-          a[3] = vb ? __ldg(pb + k2 + 4) : 0u;
+          a[0] = va ? pa[k2] : 0u;
+          a[1] = vb ? pb[k2] : 0u;
+          a[2] = va ? pa[k2 + 4] : 0u;
+          a[3] = vb ? pb[k2 + 4] : 0u;
 #pragma unroll
           for (int t = 0; t < NT; t++) {
             const uint32_t* wb = wt + (long long)t * 8 * cw + k2;
-            const uint32_t b[2] = {__ldg(wb), __ldg(wb + 4)};
+            const uint32_t b[2] = {wb[0], wb[4]};
             mma_bf16(acc[t], a, b);
           }
         }
@@ -297,7 +296,7 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool i
 
 // Weights of one slice: [P tap, x tap][channel half][R tap (descending), Cout] x 16 bytes.
 template <int COUT>
-__device__ __forceinline__ void halo_load_weights(uint32_t dst, const bf16* __restrict__ w, const HaloArgs& a, int kc,
+__device__ __forceinline__ void halo_load_weights(uint32_t dst, const bf16* w, const HaloArgs& a, int kc,
                                                   int tid) {
   for (int i = tid; i < 27 * COUT * 2; i += HT_LOADERS) {
     const int half = i & 1, co = (i >> 1) % COUT, t = (i >> 1) / COUT;  // t = (p * 3 + r) * 3 + x
@@ -309,7 +308,7 @@ __device__ __forceinline__ void halo_load_weights(uint32_t dst, const bf16* __re
 }
 
 template <int BX, bool UP>
-__device__ __forceinline__ void halo_load_slab(uint32_t dst, const bf16* __restrict__ in, const HaloArgs& a, int tile,
+__device__ __forceinline__ void halo_load_slab(uint32_t dst, const bf16* in, const HaloArgs& a, int tile,
                                                int kc, int tid) {
   constexpr int PX = BX + 2, PP = HT_P + 2;
   int t = tile;
@@ -381,7 +380,7 @@ __device__ __forceinline__ void halo_load_slab(uint32_t dst, const bf16* __restr
 
 template <int COUT, int BX, bool UP>
 __global__ void __launch_bounds__(HT_THREADS, 1)
-    conv_halo_kernel(const bf16* __restrict__ in, const bf16* __restrict__ w, const float* __restrict__ bias,
+    conv_halo_kernel(const bf16* in, const bf16* w, const float* bias,
                      bf16* __restrict__ out, const HaloArgs a, int* err) {
   constexpr int PX = BX + 2, PP = HT_P + 2, GX = BX / 8;
   constexpr int NJ = 256 / COUT < 3 ? 256 / COUT : 3;  // output planes one MMA can take (N <= 256)
@@ -583,7 +582,7 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
 template <int COUT>
 __global__ void __launch_bounds__(TC_M) conv_fwd_tma_kernel(const __grid_constant__ CUtensorMap xmap,
                                                             const __grid_constant__ CUtensorMap wmap,
-                                                            const float* __restrict__ bias, bf16* __restrict__ out,
+                                                            const float* bias, bf16* __restrict__ out,
                                                             const Geo g, const int cin, const int relu, int* err) {
   constexpr int NCOL = COUT <= 32 ? 32 : (COUT <= 64 ? 64 : 128);
   constexpr uint32_t A_LBO = TC_M * 16, B_LBO = COUT * 16;
@@ -708,7 +707,7 @@ __global__ void __launch_bounds__(TC_M) conv_fwd_tma_kernel(const __grid_constan
 }
 
 // wt[26 - tap][ci][co] = w[tap][co][ci]
-__global__ void flip_kernel(const bf16* __restrict__ w, bf16* __restrict__ wt, int cin, int cout) {
+__global__ void flip_kernel(const bf16* w, bf16* __restrict__ wt, int cin, int cout) {
   chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int total = 27 * cin * cout;
@@ -721,7 +720,7 @@ __global__ void flip_kernel(const bf16* __restrict__ w, bf16* __restrict__ wt, i
 constexpr int BW_KV = 64;  // voxels per shared-memory slab
 
 template <int CB>  // output channels / 16 (1, 2 or 4)
-__global__ void __launch_bounds__(128) conv_bwdw_kernel(const bf16* __restrict__ in, const bf16* __restrict__ dout,
+__global__ void __launch_bounds__(128) conv_bwdw_kernel(const bf16* in, const bf16* dout,
                                                         float* __restrict__ dw, const Geo g, const int cin,
                                                         const long long vox, const long long chunk) {
   chain_begin();
@@ -1013,7 +1012,7 @@ __global__ void __launch_bounds__(BT_THREADS, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ALLOC) : "memory");
 }
 
-__global__ void bias_grad_kernel(const bf16* __restrict__ dout, float* __restrict__ db, long long voxels, int c) {
+__global__ void bias_grad_kernel(const bf16* dout, float* __restrict__ db, long long voxels, int c) {
   chain_begin();
   extern __shared__ float sacc[];
   for (int k = threadIdx.x; k < c; k += blockDim.x) sacc[k] = 0.f;
@@ -1044,7 +1043,7 @@ struct Vec8 {
   float f[8];
 };
 __device__ __forceinline__ Vec8 load8(const bf16* p) {
-  const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+  const uint4 v = *reinterpret_cast<const uint4*>(p);
   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
   Vec8 r;
 #pragma unroll
@@ -1073,7 +1072,7 @@ __device__ __forceinline__ Row row_of(long long r, int d, int h) {
   return q;
 }
 
-__global__ void bias_grad8_kernel(const bf16* __restrict__ dout, float* __restrict__ db, long long groups, int c) {
+__global__ void bias_grad8_kernel(const bf16* dout, float* __restrict__ db, long long groups, int c) {
   chain_begin();
   extern __shared__ float sacc[];
   for (int k = threadIdx.x; k < c; k += blockDim.x) sacc[k] = 0.f;
@@ -1109,15 +1108,15 @@ __device__ __forceinline__ uint32_t relu_mask2(uint32_t dy, uint32_t y) {  // tw
   const float lo = __uint_as_float(y << 16), hi = __uint_as_float(y & 0xffff0000u);
   return (lo > 0.f ? dy & 0xffffu : 0u) | (hi > 0.f ? dy & 0xffff0000u : 0u);
 }
-__global__ void relu_bwd8_kernel(uint4* __restrict__ dy, const uint4* __restrict__ y, long long groups) {
+__global__ void relu_bwd8_kernel(uint4* __restrict__ dy, const uint4* y, long long groups) {
   chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= groups) return;
-  const uint4 g = dy[i], v = __ldg(y + i);
+  const uint4 g = dy[i], v = y[i];
   dy[i] = make_uint4(relu_mask2(g.x, v.x), relu_mask2(g.y, v.y), relu_mask2(g.z, v.z), relu_mask2(g.w, v.w));
 }
 
-__global__ void pool2x8_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, Geo f, int c) {
+__global__ void pool2x8_kernel(const bf16* in, bf16* __restrict__ out, Geo f, int c) {
   chain_begin();
   const int W = f.w / 2, gc = c / 8;
   const Row q = row_of(blockIdx.x, f.d / 2, f.h / 2);
@@ -1137,7 +1136,7 @@ __global__ void pool2x8_kernel(const bf16* __restrict__ in, bf16* __restrict__ o
   }
 }
 
-__global__ void pool2x8_bwd_kernel(const bf16* __restrict__ dout, bf16* __restrict__ din, Geo f, int c, int accumulate) {
+__global__ void pool2x8_bwd_kernel(const bf16* dout, bf16* __restrict__ din, Geo f, int c, int accumulate) {
   chain_begin();
   const int gc = c / 8;
   const Row q = row_of(blockIdx.x, f.d, f.h);
@@ -1161,7 +1160,7 @@ __global__ void pool2x8_bwd_kernel(const bf16* __restrict__ dout, bf16* __restri
   }
 }
 
-__global__ void up2_concat8_kernel(const uint4* __restrict__ low, const uint4* __restrict__ skip,
+__global__ void up2_concat8_kernel(const uint4* low, const uint4* skip,
                                    uint4* __restrict__ out, Geo f, int gu, int gs) {
   chain_begin();
   const int gt = gu + gs;
@@ -1170,11 +1169,11 @@ __global__ void up2_concat8_kernel(const uint4* __restrict__ low, const uint4* _
   const long long row = (long long)blockIdx.x * f.w;
   for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < f.w * gt; i += gridDim.y * blockDim.x) {
     const int x = i / gt, g = i - x * gt;
-    out[row * gt + i] = g >= gu ? __ldg(skip + (row + x) * gs + (g - gu)) : __ldg(low + (parent + x / 2) * gu + g);
+    out[row * gt + i] = g >= gu ? skip[(row + x) * gs + (g - gu)] : low[(parent + x / 2) * gu + g];
   }
 }
 
-__global__ void up2_concat8_bwd_kernel(const bf16* __restrict__ dcat, bf16* __restrict__ dlow, uint4* __restrict__ dskip,
+__global__ void up2_concat8_bwd_kernel(const bf16* dcat, bf16* __restrict__ dlow, uint4* __restrict__ dskip,
                                        Geo f, int gu, int gs, unsigned coarse_rows) {
   chain_begin();
   const int ct = (gu + gs) * 8;
@@ -1199,18 +1198,18 @@ __global__ void up2_concat8_bwd_kernel(const bf16* __restrict__ dcat, bf16* __re
   const long long row = (long long)(blockIdx.x - coarse_rows) * f.w;
   for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < f.w * gs; i += gridDim.y * blockDim.x) {
     const int x = i / gs, g = i - x * gs;
-    dskip[row * gs + i] = __ldg(reinterpret_cast<const uint4*>(dcat + (row + x) * ct) + gu + g);
+    dskip[row * gs + i] = reinterpret_cast<const uint4*>(dcat + (row + x) * ct)[gu + g];
   }
 }
 
-__global__ void relu_bwd_kernel(bf16* __restrict__ dy, const bf16* __restrict__ y, long long count) {
+__global__ void relu_bwd_kernel(bf16* __restrict__ dy, const bf16* y, long long count) {
   chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count && !(__bfloat162float(y[i]) > 0.f)) dy[i] = __float2bfloat16(0.f);
 }
 
 // ---- pooling, upsampling, concatenation ---------------------------------------------
-__global__ void pool2_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, Geo f, int c, long long count) {
+__global__ void pool2_kernel(const bf16* in, bf16* __restrict__ out, Geo f, int c, long long count) {
   chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;  // count = coarse elements
@@ -1232,7 +1231,7 @@ __global__ void pool2_kernel(const bf16* __restrict__ in, bf16* __restrict__ out
   out[i] = __float2bfloat16(s * 0.125f);
 }
 
-__global__ void pool2_bwd_kernel(const bf16* __restrict__ dout, bf16* __restrict__ din, Geo f, int c, int accumulate,
+__global__ void pool2_bwd_kernel(const bf16* dout, bf16* __restrict__ din, Geo f, int c, int accumulate,
                                  long long count) {
   chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1251,7 +1250,7 @@ __global__ void pool2_bwd_kernel(const bf16* __restrict__ dout, bf16* __restrict
   din[i] = __float2bfloat16(v);
 }
 
-__global__ void up2_concat_kernel(const bf16* __restrict__ low, const bf16* __restrict__ skip, bf16* __restrict__ out,
+__global__ void up2_concat_kernel(const bf16* low, const bf16* skip, bf16* __restrict__ out,
                                   Geo f, int cu, int cs, long long count) {
   chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1274,7 +1273,7 @@ __global__ void up2_concat_kernel(const bf16* __restrict__ low, const bf16* __re
   out[i] = low[p * cu + ch];
 }
 
-__global__ void up2_concat_bwd_low_kernel(const bf16* __restrict__ dcat, bf16* __restrict__ dlow, Geo f, int cu, int cs,
+__global__ void up2_concat_bwd_low_kernel(const bf16* dcat, bf16* __restrict__ dlow, Geo f, int cu, int cs,
                                           long long count) {
   chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1297,7 +1296,7 @@ __global__ void up2_concat_bwd_low_kernel(const bf16* __restrict__ dcat, bf16* _
   dlow[i] = __float2bfloat16(s);
 }
 
-__global__ void up2_concat_bwd_skip_kernel(const bf16* __restrict__ dcat, bf16* __restrict__ dskip, int cu, int cs,
+__global__ void up2_concat_bwd_skip_kernel(const bf16* dcat, bf16* __restrict__ dskip, int cu, int cs,
                                            long long count) {
   chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1311,8 +1310,8 @@ __global__ void up2_concat_bwd_skip_kernel(const bf16* __restrict__ dcat, bf16* 
 // of voxels serialised 65,536 of them on one address).  PACKED: 16 channels of which 4 have
 // targets, 16-byte aligned.
 template <bool PACKED>
-__global__ void __launch_bounds__(256) mse_kernel(const bf16* __restrict__ out, const float* __restrict__ target,
-                                                  const uint8_t* __restrict__ mask, const float* __restrict__ cw,
+__global__ void __launch_bounds__(256) mse_kernel(const bf16* out, const float* target,
+                                                  const uint8_t* mask, const float* cw,
                                                   bf16* __restrict__ dout, double* loss, long long voxels, int cpad,
                                                   int ct, double count) {
   chain_begin();
@@ -1323,8 +1322,8 @@ __global__ void __launch_bounds__(256) mse_kernel(const bf16* __restrict__ out, 
     if (PACKED) {
       uint4 lo = make_uint4(0u, 0u, 0u, 0u);
       if (on) {
-        const uint2 o = __ldg(reinterpret_cast<const uint2*>(out + v * 16));
-        const float4 t = __ldg(reinterpret_cast<const float4*>(target + v * 4));
+        const uint2 o = *reinterpret_cast<const uint2*>(out + v * 16);
+        const float4 t = *reinterpret_cast<const float4*>(target + v * 4);
         const float d[4] = {__uint_as_float(o.x << 16) - t.x, __uint_as_float(o.x & 0xffff0000u) - t.y,
                             __uint_as_float(o.y << 16) - t.z, __uint_as_float(o.y & 0xffff0000u) - t.w};
         float gr[4];
@@ -1362,7 +1361,7 @@ __global__ void __launch_bounds__(256) mse_kernel(const bf16* __restrict__ out, 
   }
 }
 
-__global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
+__global__ void adam_kernel(float* __restrict__ w, const float* g, float* __restrict__ m,
                             float* __restrict__ v, bf16* __restrict__ wb, long long count, float lr, float b1, float b2,
                             float eps, float c1, float c2) {
   chain_begin();
@@ -1378,20 +1377,20 @@ __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, 
   if (wb) wb[i] = __float2bfloat16(wi);
 }
 
-__global__ void to_bf16_kernel(const float* __restrict__ x, bf16* __restrict__ y, long long count) {
+__global__ void to_bf16_kernel(const float* x, bf16* __restrict__ y, long long count) {
   chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) y[i] = __float2bfloat16(x[i]);
 }
 
-__global__ void from_bf16_kernel(const bf16* __restrict__ x, float* __restrict__ y, long long count) {
+__global__ void from_bf16_kernel(const bf16* x, float* __restrict__ y, long long count) {
   chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) y[i] = __bfloat162float(x[i]);
 }
 
 // out[0] += sum (a - b)^2, out[1] += sum a^2 (FP64), for steady-state tests.
-__global__ void diff_norms_kernel(const float* __restrict__ a, const float* __restrict__ b, long long count,
+__global__ void diff_norms_kernel(const float* a, const float* b, long long count,
                                   double* out) {
   chain_begin();
   double d2 = 0.0, a2 = 0.0;
@@ -1463,7 +1462,7 @@ __global__ void features_kernel(bf16* __restrict__ out, int nx, int ny, int nz, 
 // out (n, 4, d, h, w) FP32 (+)= weight * the first four channels of y (n, d, h, w, 16),
 // read from the mirror image in y and/or z, with the mirrored velocity components
 // (channel 2 = u_y, 3 = u_z) negated: undoes a reflection of the input.
-__global__ void unpack_fields_kernel(const bf16* __restrict__ y, float* __restrict__ out, Geo g, int flip_y, int flip_z,
+__global__ void unpack_fields_kernel(const bf16* y, float* __restrict__ out, Geo g, int flip_y, int flip_z,
                                      float weight, int accumulate, long long count) {
   chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
