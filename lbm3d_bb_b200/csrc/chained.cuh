@@ -22,6 +22,7 @@ __device__ __forceinline__ void chain_begin() {
   chain_wait();
 }
 
+// Leaves a refused launch in the runtime's last error too, for callers that ask there.
 template <class... P, class... A>
 inline cudaError_t launch_chained_smem(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                                        A&&... args) {
@@ -37,9 +38,13 @@ inline cudaError_t launch_chained_smem(void (*kernel)(P...), dim3 grid, dim3 blo
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
+// A launch that is refused is reported by the return value alone: the runtime's last error, which
+// whoever launches next asks for, is taken back.
 template <class... P, class... A>
 inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A&&... args) {
-  return launch_chained_smem(kernel, grid, block, 0, s, static_cast<A&&>(args)...);
+  const cudaError_t e = launch_chained_smem(kernel, grid, block, 0, s, static_cast<A&&>(args)...);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e;
 }
 
 }  // namespace lbm
