@@ -35,6 +35,8 @@ bool pose_equal(const lbm_pose& a, const lbm_pose& b) { return std::memcmp(&a, &
 
 }  // namespace
 
+constexpr int MAX_GRID_Y = 65535;  // blocks along y of a launch
+
 struct lbm_ctx {
   lbm_config cfg{};
   int device = 0;
@@ -100,8 +102,9 @@ struct lbm_ctx {
     return dim3((unsigned)((g.nx + bx - 1) / bx), (unsigned)((g.ny + by - 1) / by), (unsigned)g.nz);
   }
   // kernels that only stream a row's nodes (export, initialisation): rows longer than 128 in
-  // blocks of 128 x 1 (FP64 343x220x218 export 435 us, 452 in blocks of 32 x 4 on B200)
-  dim3 row_block() const { return g.nx > 128 ? dim3(128, 1, 1) : block(); }
+  // blocks of 128 x 1 (FP64 343x220x218 export 435 us, 452 in blocks of 32 x 4 on B200), as long
+  // as a grid has that many blocks along y
+  dim3 row_block() const { return g.nx > 128 && g.ny <= MAX_GRID_Y ? dim3(128, 1, 1) : block(); }
   dim3 row_grid() const {
     const dim3 b = row_block();
     return dim3((unsigned)((g.nx + b.x - 1) / b.x), (unsigned)((g.ny + b.y - 1) / b.y), (unsigned)g.nz);
@@ -786,7 +789,9 @@ int32_t lbm_create(const lbm_config* cfg, int32_t device, lbm_ctx** out) {
     // FP32 and FP16-deviation storage (faster on B200: +2 % and +16 % on the 512^3 porous
     // box), not for FP64 (15 % slower); LBM3D_PAIR=1 / 0 forces it on / off
     const char* env = std::getenv("LBM3D_PAIR");
-    const bool fits = !c->ref && !c->tma && cfg->nx % 128 == 0 && c->g.per[0] && c->g.per[1] &&
+    // (its smallest blocks take one row: boxes with more rows than a grid has blocks along y take
+    // aa_rows_kernel, which numbers its blocks along x)
+    const bool fits = !c->ref && !c->tma && cfg->nx % 128 == 0 && cfg->ny <= MAX_GRID_Y && c->g.per[0] && c->g.per[1] &&
                       (c->g.per[2] || halo_only(c));
     const bool wanted = env ? env[0] == '1' : cfg->storage != LBM_STORE_FP64;
     c->pair = fits && wanted;
