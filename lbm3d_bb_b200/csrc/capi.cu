@@ -79,6 +79,7 @@ struct lbm_ctx {
   int bx = 0, by = 0;
   bool pair = false;  // FP16 pair kernel (see aa_pair_kernel)
   bool rows = false;  // two cells per thread, any even row length and any faces (aa_rows_kernel)
+  bool rows_forced = false;  // LBM3D_PAIR=1
   bool quad = false;  // FP16-deviation on the four-cell kernels
   bool xshuffle = false;  // FP32 odd phase on aa_pair_odd_kernel
   bool octo = false;  // FP16-deviation even phase on aa_octo_even_kernel
@@ -799,9 +800,10 @@ int32_t lbm_create(const lbm_config* cfg, int32_t device, lbm_ctx** out) {
     // smaller boxes do not fill the GPU with half the threads (B200, us per step, one cell /
     // rows, FP32: channel 96x48x48 11.3 / 11.7, 128x96x96 39 / 40, 160x96x96 49.0 / 49.0,
     // 192x120x120 86 / 82, 384x192x192 411 / 374; FP16 deviations 160x96x96 43.1 / 41.8).
-    // LBM3D_PAIR=1 / 0 forces it on / off
+    // LBM3D_PAIR=1 / 0 forces it on / off, also for boxes with a moving body (lbm_step)
     c->rows = !c->ref && !c->tma && !c->pair && cfg->nx % 2 == 0 && cfg->nx >= 4 && cfg->storage != LBM_STORE_FP64 &&
               (env ? env[0] == '1' : c->g.N >= 1400000);
+    c->rows_forced = c->rows && env;
     // four cells per thread in the FP16-deviation even phase (aa_quad_even_kernel);
     // LBM3D_QUAD=0 keeps the pair kernels
     const char* q = std::getenv("LBM3D_QUAD");
@@ -1093,7 +1095,7 @@ int32_t lbm_step(lbm_ctx* c, int32_t nsteps) {
       // FP32 TRT 192x96x96 87 / 72, BGK 280x150x150 218 / 216, 331x160x160 289 / 298; FP16
       // TRT 192x96x96 75 / 63, 331x160x160 273 / 281, BGK 256x128x128 130 / 146)
       const bool bgk16 = c->cfg.storage == LBM_STORE_FP16DEV && !trt;
-      p.move = c->has_moving && has_faces(c) && c->g.N < (bgk16 ? 2000000 : 6000000);
+      p.move = c->has_moving && has_faces(c) && !c->rows_forced && c->g.N < (bgk16 ? 2000000 : 6000000);
       p.pair = c->pair ? 1 : (c->rows && !p.move ? 2 : 0);
       p.quad = c->pair && c->quad ? (c->swapped ? (c->quad_odd ? 1 : 0) : (c->octo ? 2 : 1)) : 0;
       p.xshuffle = c->pair && c->xshuffle ? 1 : 0;

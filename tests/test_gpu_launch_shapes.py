@@ -1,10 +1,13 @@
-"""Block shapes that a program sets (lbm_set_launch): a refused launch is an error of that call and
-of no later one."""
+"""Block shapes that a program sets (lbm_set_launch, LBM3D_BLOCK) and the kernels that serve them: a
+refused launch is an error of that call and of no later one, and boxes with very many rows run."""
+import re
+
 import numpy as np
 import pytest
 
 from lbm3d_bb_b200 import Domain
 from lbm3d_bb_b200._capi import LbmError
+from tests import cases
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +65,27 @@ def test_more_rows_than_a_grid_has_blocks(gpu, storage, monkeypatch):
     assert (out[0][1:] != 0).any()
     tol = 1e-6 if storage == "fp32" else 2e-4  # a rounding of an FP16 deviation of order 0.1
     assert (out[0] - out[1]).abs().max().item() <= tol
+
+
+def _step_kernels(d, steps=2):
+    """Names of the step kernels that `steps` steps launch (even and odd phase)."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        d.step(steps)
+        torch.cuda.synchronize()
+    names = {re.sub(r".*\b(\w+_kernel)\b.*", r"\1", e.name) for e in p.events() if "_kernel" in e.name}
+    return names
+
+
+@pytest.mark.parametrize("pair,kernel", [(None, "aa_step_kernel"), ("0", "aa_step_kernel"), ("1", "aa_rows_kernel")])
+def test_pair_variable_holds_with_a_moving_body(gpu, monkeypatch, pair, kernel):
+    if pair is not None:
+        monkeypatch.setenv("LBM3D_PAIR", pair)
+    d = cases.moving_sphere_trt(Domain, storage="fp32")
+    try:
+        d.update_body(*cases.sphere_pose(d, 1))
+        assert _step_kernels(d) - {"body_flags_kernel"} == {kernel}
+    finally:
+        d.close()
