@@ -193,8 +193,11 @@ int32_t lbm_set_stream(lbm_ctx* ctx, void* stream);
 int32_t lbm_synchronize(lbm_ctx* ctx);
 /* Bytes of device memory the context holds. */
 int64_t lbm_device_bytes(const lbm_ctx* ctx);
-/* Thread-block shape of the step kernels (bx along x, by along y; bx*by a
- * multiple of 32, at most 256).  Chosen per lattice size by the autotuner; no
+/* Thread-block shape of the one-cell step kernels (bx along x, by along y; bx*by a
+ * multiple of 32, at most 256).  Kernels with several cells per thread have shapes of
+ * their own: fully periodic boxes with nx a multiple of 128 keep theirs, other boxes
+ * with even nx leave theirs for the one-cell kernel when a shape is set that differs
+ * from the one the library chose.  Chosen per lattice size by the autotuner; no
  * reference counterpart (CUDA.jl launches 256 threads, Collision.jl:95-96). */
 int32_t lbm_set_launch(lbm_ctx* ctx, int32_t bx, int32_t by);
 int32_t lbm_get_launch(const lbm_ctx* ctx, int32_t* bx, int32_t* by);

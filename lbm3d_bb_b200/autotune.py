@@ -3,7 +3,8 @@
 For a lattice size, storage, collision and face set, every candidate block shape
 (bx threads along x, by rows; whole warps, at most 256 threads) is timed on the
 device with CUDA events over a few steps of the caller's own domain, and the fastest
-is applied with ``lbm_set_launch``.  Results are cached in a JSON file keyed by GPU
+is applied with ``lbm_set_launch``.  The shape that the library chooses itself is among
+them and stands for the kernel that it chooses with it.  Results are cached in a JSON file keyed by GPU
 name and configuration (``$LBM3D_TUNE_CACHE``, default
 ``~/.cache/lbm3d/launch_shapes.json``), so a shape is measured once per machine.
 
@@ -20,6 +21,7 @@ from typing import Callable, Optional, Sequence
 
 from . import abi
 
+KERNELS = 2  # raised when a shape stands for another kernel: shapes measured before are measured again
 FACE_NAMES = {v: k for k, v in abi.FACES.items()}
 
 
@@ -31,7 +33,7 @@ def config_key(d, device_name: str) -> str:
     c = d.cfg
     faces = ",".join(FACE_NAMES.get(int(c.face[k]), str(int(c.face[k]))) for k in range(6))
     return (f"{device_name}|{c.nx}x{c.ny}x{c.nz}|storage={int(c.storage)}|coll={int(c.collision)}|"
-            f"mode={int(c.mode)}|faces={faces}")
+            f"mode={int(c.mode)}|faces={faces}|kernels={KERNELS}")
 
 
 def candidates(nx: int) -> list[tuple[int, int]]:
@@ -43,6 +45,9 @@ def candidates(nx: int) -> list[tuple[int, int]]:
         for threads in (128, 256):
             if threads % bx == 0:
                 out.append((bx, threads // bx))
+    padded = -(-nx // 32) * 32
+    if padded <= 128:  # a padded row
+        out.append((padded, 128 // padded))
     if nx <= 256:  # whole rows, as many as fit whole warps (the default heuristic's family)
         for by in range(1, 257):
             if nx * by > 256:

@@ -77,6 +77,7 @@ struct lbm_ctx {
   bool any_body = false;
   // launch shape
   int bx = 0, by = 0;
+  int own_bx = 0, own_by = 0;  // the shape default_block chose
   bool pair = false;  // FP16 pair kernel (see aa_pair_kernel)
   bool rows = false;  // two cells per thread, any even row length and any faces (aa_rows_kernel)
   bool rows_forced = false;  // LBM3D_PAIR=1
@@ -99,6 +100,9 @@ struct lbm_ctx {
     return fail(LBM_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   }
   dim3 block() const { return dim3((unsigned)bx, (unsigned)by, 1); }
+  // aa_rows_kernel has a block shape of its own: a program that sets another shape than the
+  // library's (lbm_set_launch, LBM3D_BLOCK) gets the one-cell kernel with it
+  bool rows_now() const { return rows && (rows_forced || (bx == own_bx && by == own_by)); }
   dim3 grid() const {
     return dim3((unsigned)((g.nx + bx - 1) / bx), (unsigned)((g.ny + by - 1) / by), (unsigned)g.nz);
   }
@@ -136,6 +140,8 @@ void default_block(lbm_ctx* c) {
     bx = (nx + 31) / 32 * 32;
     by = std::max(1, 128 / bx);
   }
+  c->own_bx = bx;
+  c->own_by = by;
   const char* env = std::getenv("LBM3D_BLOCK");
   if (env) {
     int ex = 0, ey = 0;
@@ -1096,7 +1102,7 @@ int32_t lbm_step(lbm_ctx* c, int32_t nsteps) {
       // TRT 192x96x96 75 / 63, 331x160x160 273 / 281, BGK 256x128x128 130 / 146)
       const bool bgk16 = c->cfg.storage == LBM_STORE_FP16DEV && !trt;
       p.move = c->has_moving && has_faces(c) && !c->rows_forced && c->g.N < (bgk16 ? 2000000 : 6000000);
-      p.pair = c->pair ? 1 : (c->rows && !p.move ? 2 : 0);
+      p.pair = c->pair ? 1 : (c->rows_now() && !p.move ? 2 : 0);
       p.quad = c->pair && c->quad ? (c->swapped ? (c->quad_odd ? 1 : 0) : (c->octo ? 2 : 1)) : 0;
       p.xshuffle = c->pair && c->xshuffle ? 1 : 0;
       if (c->tma) {

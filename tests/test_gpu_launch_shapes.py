@@ -1,5 +1,6 @@
 """Block shapes that a program sets (lbm_set_launch, LBM3D_BLOCK) and the kernels that serve them: a
-refused launch is an error of that call and of no later one, and boxes with very many rows run."""
+refused launch is an error of that call and of no later one, boxes with very many rows run, and a
+set shape is the shape of the step."""
 import re
 
 import numpy as np
@@ -10,6 +11,8 @@ from lbm3d_bb_b200._capi import LbmError
 from tests import cases
 
 pytestmark = pytest.mark.gpu
+
+CHANNEL = ("inlet", "pressure", "wall", "wall", "wall", "wall")
 
 
 def _tall(storage="fp64"):
@@ -77,6 +80,59 @@ def _step_kernels(d, steps=2):
         torch.cuda.synchronize()
     names = {re.sub(r".*\b(\w+_kernel)\b.*", r"\1", e.name) for e in p.events() if "_kernel" in e.name}
     return names
+
+
+def test_a_set_shape_selects_the_one_cell_kernel(gpu):
+    """Of boxes whose step has a kernel with a shape of its own; the library's shape gives it back."""
+    d = Domain(160, 96, 96, storage="fp32", faces=CHANNEL, omega_p=1.3, face_u=[(0.03, 0.0, 0.0)] + [(0.0, 0.0, 0.0)] * 5)
+    d.add_sphere((40.0, 48.0, 48.0), 9.0)
+    d.init_equilibrium()
+    try:
+        own = d.launch()
+        assert _step_kernels(d) == {"aa_rows_kernel"}
+        for shape in ((32, 8), (160, 1)):
+            assert shape != own
+            d.set_launch(*shape)
+            assert d.launch() == shape and _step_kernels(d) == {"aa_step_kernel"}
+        d.set_launch(*own)
+        assert _step_kernels(d) == {"aa_rows_kernel"}
+    finally:
+        d.close()
+
+
+def test_block_variable_selects_the_one_cell_kernel(gpu, monkeypatch):
+    for block, pair, kernel in (("32,8", None, "aa_step_kernel"), ("32,8", "1", "aa_rows_kernel"), (None, None, "aa_rows_kernel")):
+        for name, value in (("LBM3D_BLOCK", block), ("LBM3D_PAIR", pair)):
+            if value is None:
+                monkeypatch.delenv(name, raising=False)
+            else:
+                monkeypatch.setenv(name, value)
+        d = Domain(160, 96, 96, storage="fp32", faces=CHANNEL, omega_p=1.3)
+        d.init_equilibrium()
+        try:
+            assert _step_kernels(d) == {kernel}
+        finally:
+            d.close()
+
+
+def test_the_tuner_times_the_librarys_own_shape(gpu, tmp_path, monkeypatch):
+    """Rows that fit no whole warps: the padded row is the library's shape and a candidate; when it
+    is the fastest, the kernel that goes with it stays."""
+    from lbm3d_bb_b200 import autotune
+
+    monkeypatch.setenv("LBM3D_TUNE_CACHE", str(tmp_path / "shapes.json"))
+    for nx in (70, 160, 96, 34):
+        d = Domain(nx, 8, 8, storage="fp32")
+        assert d.launch() in autotune.candidates(nx)
+        d.close()
+    d = Domain(160, 96, 96, storage="fp32", faces=CHANNEL, omega_p=1.3)
+    d.init_equilibrium()
+    own = d.launch()
+    try:
+        got = autotune.tune(d, timer=lambda: 0.0 if d.launch() == own else 1.0)
+        assert got == own and _step_kernels(d) == {"aa_rows_kernel"}
+    finally:
+        d.close()
 
 
 @pytest.mark.parametrize("pair,kernel", [(None, "aa_step_kernel"), ("0", "aa_step_kernel"), ("1", "aa_rows_kernel")])
