@@ -18,7 +18,8 @@ struct RefT<double> {
 // (the compiler must keep x * 0).  Opposite directions share their sums: every term of d is the
 // same as or the exact negative of that of opp(d).  Same bits, but for the sign of a zero, with
 // less than half the arithmetic, which bounds the step (B200, D3Q19 TRT 480x240x4 with the
-// flags of a moving cylinder: 32.2 -> 29.9 us per step).
+// flags of a moving cylinder: 32.2 -> 29.9 us per step).  Where a term is not finite the
+// reference's product with zero makes the sum NaN: ref_moments and ref_collide see to that.
 template <class T>
 __device__ __forceinline__ void ref_add(T& s, int c, T f) {
   if (c > 0) s += f;
@@ -60,6 +61,12 @@ __device__ __forceinline__ void ref_moments(const T* S, T& rho, T& u, T& v, T& w
   u = mx / r;
   v = my / r;
   w = mz / r;
+  if (!isfinite(r)) {
+    bool bad = false;
+#pragma unroll
+    for (int d = 0; d < Q; d++) bad = bad || !isfinite(S[d]);
+    if (bad) u = v = w = r - r;  // infinite or NaN momenta over an infinite or NaN density
+  }
 }
 
 // BGK_collision!_gpu (Collision.jl:229-238) and TRT_collision!_gpu
@@ -67,7 +74,8 @@ __device__ __forceinline__ void ref_moments(const T* S, T& rho, T& u, T& v, T& w
 template <class T, bool TRT>
 __device__ __forceinline__ void ref_collide(const T* S, T* F, T rho, T ux, T uy, T uz, T om_p, T om_m) {
   const T u2 = ux * ux + uy * uy + uz * uz;
-  const T u2t = T(0.5) * u2 * T(3);
+  T u2t = T(0.5) * u2 * T(3);
+  if (isinf(u2t)) u2t += (ux - ux) + (uy - uy) + (uz - uz);  // NaN where a component is infinite
 #pragma unroll
   for (int d = 0; d < Q; d += 2) {  // d, opp(d) = d + 1; the rest direction is the last one
     const T wr = RefT<T>::W(d) * rho;
