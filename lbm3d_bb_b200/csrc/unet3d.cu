@@ -1492,18 +1492,16 @@ __global__ void unpack_fields_kernel(const bf16* y, float* __restrict__ out, Geo
 // copy engine issues one request per 16-byte row, and 27 times per voxel)
 int g_engine = 2;
 
-// cuTensorMapEncodeTiled from the driver (fetched once, no link against libcuda).
+// cuTensorMapEncodeTiled from the driver (fetched once, no link against libcuda); threads that ask
+// at the same time wait for the one that fetches it.
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
+  static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
-  }
+    const bool found = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+                       q == cudaDriverEntryPointSuccess;
+    return found ? (PFN_cuTensorMapEncodeTiled_v12000)p : nullptr;
+  }();
   return fn;
 }
 
