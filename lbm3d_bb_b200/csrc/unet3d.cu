@@ -1505,6 +1505,24 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
+// Tensor map of BF16 tiles (no swizzle, zero fill).  The encoder fails on a thread that has not
+// used the device yet and so has no current context (the kernel launch that follows would give
+// it one): such a thread gets the runtime's and tries once more.
+bool encode_tiles(CUtensorMap& map, int rank, const void* p, const cuuint64_t* dim, const cuuint64_t* str,
+                  const cuuint32_t* box) {
+  const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+  if (!enc) return false;
+  const cuuint32_t one[5] = {1, 1, 1, 1, 1};
+  const auto encode = [&] {
+    return enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(p), dim, str, box, one,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  if (encode()) return true;
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess && encode();
+}
+
 // The TMA-fed kernel takes tiles of 128 voxels that are whole rows or part of one row.
 bool tma_tiles_fit(int h, int w) {
   if (w >= TC_M) return w % TC_M == 0;
@@ -1658,17 +1676,13 @@ int halo_conv(const bf16* in, const bf16* w, const float* bias, bf16* out, const
 // Tensor map over channels-last activations seen as (8 channels, x, ...): the 8-channel groups
 // are an axis of their own, before (group_first) or after y, and z runs over the whole batch.
 bool activation_map(CUtensorMap& map, const void* p, const Geo& g, int c, bool group_first, int bx, int by, int bg) {
-  PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-  if (!enc || (long long)g.n * g.d > 0x7fffffffLL) return false;
+  if ((long long)g.n * g.d > 0x7fffffffLL) return false;
   const cuuint64_t row = (cuuint64_t)g.w * c * 2;
   const cuuint64_t ng = (cuuint64_t)c / 8, nh = (cuuint64_t)g.h;
   const cuuint64_t dim[5] = {8, (cuuint64_t)g.w, group_first ? ng : nh, group_first ? nh : ng, (cuuint64_t)g.n * g.d};
   const cuuint64_t str[4] = {(cuuint64_t)c * 2, group_first ? 16 : row, group_first ? row : 16, row * nh};
   const cuuint32_t box[5] = {8, (cuuint32_t)bx, (cuuint32_t)(group_first ? bg : by), (cuuint32_t)(group_first ? by : bg), 1};
-  const cuuint32_t one[5] = {1, 1, 1, 1, 1};
-  return enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(p), dim, str, box, one,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return encode_tiles(map, 5, p, dim, str, box);
 }
 
 // Tile of the weight gradient: y rows and z planes of a block's slab.  The model counts cycles
@@ -1776,7 +1790,7 @@ int32_t nn_conv3d_fwd(const void* in, const void* w, const float* bias, void* ou
   if (g_engine != 0) {
     int* err = tc_err_ptr();
     if (!err) return fail("nn_conv3d_fwd: no device address for the error word");
-    PFN_cuTensorMapEncodeTiled_v12000 enc = g_engine == 3 ? tensor_map_encoder() : nullptr;
+    const bool enc = g_engine == 3 && tensor_map_encoder();
     if (enc && tma_tiles_fit(h, wd) && cin % 16 == 0) {
       CUtensorMap xmap, wmap;
       const cuuint64_t xdim[5] = {(cuuint64_t)cin, (cuuint64_t)wd, (cuuint64_t)h, (cuuint64_t)d, (cuuint64_t)n};
@@ -1784,17 +1798,11 @@ int32_t nn_conv3d_fwd(const void* in, const void* w, const float* bias, void* ou
                                   (cuuint64_t)d * h * wd * cin * 2};
       const int bw = wd < TC_M ? wd : TC_M;
       const cuuint32_t xbox[5] = {8, (cuuint32_t)bw, (cuuint32_t)(TC_M / bw), 1, 1};
-      const cuuint32_t one[5] = {1, 1, 1, 1, 1};
       const cuuint64_t wdim[3] = {(cuuint64_t)cin, (cuuint64_t)cout, 27};
       const cuuint64_t wstr[2] = {(cuuint64_t)cin * 2, (cuuint64_t)cout * cin * 2};
       const cuuint32_t wbox[3] = {8, (cuuint32_t)cout, 1};
-      CUresult r1 = enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(in), xdim, xstr, xbox, one,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      CUresult r2 = enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(w), wdim, wstr, wbox, one,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      if (r1 != CUDA_SUCCESS || r2 != CUDA_SUCCESS) return fail("nn_conv3d_fwd: tensor map encoding failed (%d, %d)", (int)r1, (int)r2);
+      if (!encode_tiles(xmap, 5, in, xdim, xstr, xbox) || !encode_tiles(wmap, 3, w, wdim, wstr, wbox))
+        return fail("nn_conv3d_fwd: tensor map encoding failed");
       const unsigned tgrid = (unsigned)((long long)n * d * (h / (TC_M / bw)) * (wd / bw));
       switch (cout) {
         case 16: launch_chained_smem(conv_fwd_tma_kernel<16>, tgrid, TC_M, 0, s, xmap, wmap, bias, O, g, cin, relu,

@@ -54,3 +54,10 @@ def test_first_weight_gradients_of_several_threads(gpu, run):
     r = subprocess.run([sys.executable, "-c", FIRST_CALLS], cwd=ROOT, capture_output=True, text=True, timeout=300,
                        env={**os.environ, "THREADS": "known"})
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_weight_gradients_of_threads_new_to_the_device(gpu):
+    """The network's call is the first that these threads make: no context is current yet."""
+    r = subprocess.run([sys.executable, "-c", FIRST_CALLS], cwd=ROOT, capture_output=True, text=True, timeout=300,
+                       env={**os.environ, "THREADS": "new"})
+    assert r.returncode == 0, r.stderr[-2000:]
