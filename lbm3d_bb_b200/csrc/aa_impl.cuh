@@ -654,6 +654,12 @@ __device__ __noinline__ void moving_links_call(const AAParams& p, const int x, c
     double t = (double)pst[o] + (double)v;
     if (SP::DEV) t += 2.0 * (double)(wgt<C>(o) * C(p.rho0));
     pst[o] = v;
+    if (!isfinite(t)) {  // a lost node's links make every component NaN that they do not point along
+      fx += t * cx(o);
+      fy += t * cy(o);
+      fz += t * cz(o);
+      continue;
+    }
     if (cx(o) > 0) fx += t;
     if (cx(o) < 0) fx -= t;
     if (cy(o) > 0) fy += t;
