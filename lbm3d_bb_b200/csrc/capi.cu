@@ -121,18 +121,26 @@ namespace {
 void default_block(lbm_ctx* c) {
   // rows of the box across threadIdx.x; whole warps, at most 256 threads (the step
   // kernels' launch bound).  Rows that fit no such shape are padded to 32 lanes.  Rows longer
-  // than 128 take blocks of 128 threads, 32, 64 or 128 wide.  32 x 4 is the fastest wherever
-  // faces or the reference step leave work to single lanes (B200, us per step against 128 x 1:
-  // FP32 channel 160x96x96 48.6 / 58.5, 384-wide equal, FP64 331x120x119 266 / 278, reference
-  // 480x240x4 26.6 / 28.7); fully periodic boxes and, from 4 M cells, others too take the
-  // widest of the three that pads least (FP32 192x96x96 62.4 / 68.7, FP64 383x120x120 128 x 1
-  // 318.7, 32 x 4 322.1, FP64 channel 225x205x200 549, 32 x 4 580).
+  // than 128 take blocks of 128 threads, 128 x 1, 64 x 2 or 32 x 4, of those that pad least
+  // (within 3 %): 32 x 4 first, the fastest wherever faces or the reference step leave work to
+  // single lanes (B200, us per step against 128 x 1: FP32 channel 160x96x96 48.6 / 58.5, 384-wide
+  // equal, FP64 331x120x119 266 / 278, reference 480x240x4 26.6 / 28.7); in fully periodic boxes
+  // and, from 4 M cells, others too the widest first (FP32 192x96x96 62.4 / 68.7, FP64
+  // 383x120x120 128 x 1 318.7, 32 x 4 322.1, FP64 channel 225x205x200 549, 32 x 4 580).  Few rows
+  // count as much as few lanes (32 x 4 / 64 x 2 / 128 x 1: FP64 channel 161x2x1242 33.1 / 23.8 /
+  // 27.5, reference 161x2x13043 310 / 208 / 244, FP32 TRT channel 161x5x496 19.7 / 17.5 / 18.2).
   const int nx = c->g.nx;
   int bx = nx <= 128 ? nx : 128;
   if (nx > 128) {
     const bool widest = !c->ref && ((c->g.per[0] && c->g.per[1] && c->g.per[2]) || c->g.N >= 4000000);
-    for (int w : {64, 32})
-      if (!widest || (nx + w - 1) / w * w < (nx + bx - 1) / bx * bx) bx = w;
+    const auto threads = [&](int w) {  // of one z plane
+      const int rows = 128 / w;
+      return (long long)((nx + w - 1) / w * w) * ((c->g.ny + rows - 1) / rows * rows);
+    };
+    const long long least = std::min(threads(128), std::min(threads(64), threads(32)));
+    bx = 0;
+    for (int w : {widest ? 128 : 32, 64, widest ? 32 : 128})
+      if (!bx && threads(w) * 100 <= least * 103) bx = w;
   }
   int by = std::max(1, 128 / bx);
   while ((bx * by) % 32 != 0 && bx * (by + 1) <= 256) by++;

@@ -145,3 +145,17 @@ def test_pair_variable_holds_with_a_moving_body(gpu, monkeypatch, pair, kernel):
         assert _step_kernels(d) - {"body_flags_kernel"} == {kernel}
     finally:
         d.close()
+
+
+@pytest.mark.parametrize("shape,block", [((161, 2, 40), (64, 2)), ((161, 5, 40), (64, 2)), ((161, 6, 40), (64, 2)),
+                                         ((161, 12, 40), (32, 4)), ((1000, 1, 3), None), ((384, 3, 9), (128, 1)), ((300, 200, 3), (32, 4))])
+def test_blocks_have_no_more_rows_than_boxes_fill(gpu, shape, block):
+    if shape[1] < 2:
+        with pytest.raises(LbmError):
+            Domain(*shape, storage="fp64", faces=CHANNEL)
+        return
+    d = Domain(*shape, storage="fp64", faces=CHANNEL)
+    try:
+        assert d.launch() == block
+    finally:
+        d.close()
