@@ -814,9 +814,19 @@ int32_t lbm_create(const lbm_config* cfg, int32_t device, lbm_ctx** out) {
     // smaller boxes do not fill the GPU with half the threads (B200, us per step, one cell /
     // rows, FP32: channel 96x48x48 11.3 / 11.7, 128x96x96 39 / 40, 160x96x96 49.0 / 49.0,
     // 192x120x120 86 / 82, 384x192x192 411 / 374; FP16 deviations 160x96x96 43.1 / 41.8).
+    // With faces, rows on a y or z end take the one-cell path there, one cell after the other:
+    // boxes where more than an eighth of the rows (FP16 deviations: a quarter) lie on one keep one
+    // cell per thread (rows / one cell, channels of 1.5 M cells, share of such rows: FP32
+    // 434x434x8 0.25 1.11, 354x354x12 0.17 1.05, 252x252x24 0.09 1.01, 614x614x4 0.50 1.23; FP16
+    // 0.50 1.10, 10416x12x12 0.31 1.06, 0.25 0.94; of 10 M cells FP32 0.25 1.02, 0.13 0.94).
+    // So do boxes below 6 M cells with rows of ten cells or less: a warp spans many rows there, and
+    // one link or face among them costs all its lanes (channels with a sphere, FP16: 4x600x600
+    // 56.1 / 45.6, 8x434x434 51.4 / 47.6, 16x320x300 46.3 / 47.7, 4x1500x1000 164 / 182).
     // LBM3D_PAIR=1 / 0 forces it on / off, also for boxes with a moving body (lbm_step)
+    const double inner = (double)std::max(cfg->ny - 2, 0) * std::max(cfg->nz - 2, 0) / ((double)cfg->ny * cfg->nz);
+    const bool ends_fit = !has_faces(c) || halo_only(c) || inner >= (cfg->storage == LBM_STORE_FP32 ? 0.875 : 0.75);
     c->rows = !c->ref && !c->tma && !c->pair && cfg->nx % 2 == 0 && cfg->nx >= 4 && cfg->storage != LBM_STORE_FP64 &&
-              (env ? env[0] == '1' : c->g.N >= 1400000);
+              (env ? env[0] == '1' : c->g.N >= 1400000 && ends_fit && (cfg->nx >= 12 || c->g.N >= 6000000));
     c->rows_forced = c->rows && env;
     // four cells per thread in the FP16-deviation even phase (aa_quad_even_kernel);
     // LBM3D_QUAD=0 keeps the pair kernels

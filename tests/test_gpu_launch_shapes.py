@@ -147,6 +147,27 @@ def test_pair_variable_holds_with_a_moving_body(gpu, monkeypatch, pair, kernel):
         d.close()
 
 
+@pytest.mark.parametrize("shape,faces,storage,kernel", [
+    ((614, 614, 4), "channel", "fp32", "aa_step_kernel"),     # half of the rows on a z end
+    ((614, 614, 4), "channel", "fp16dev", "aa_step_kernel"),
+    ((614, 614, 4), "periodic", "fp32", "aa_rows_kernel"),
+    ((354, 354, 12), "channel", "fp32", "aa_step_kernel"),    # a sixth
+    ((354, 354, 12), "channel", "fp16dev", "aa_rows_kernel"),
+    ((1200, 1200, 1), "channel", "fp32", "aa_step_kernel"),   # all of them
+    ((252, 252, 24), "channel", "fp32", "aa_rows_kernel"),
+    ((4, 600, 600), "channel", "fp16dev", "aa_step_kernel"),  # rows of a few cells
+    ((12, 400, 360), "channel", "fp16dev", "aa_rows_kernel"),
+    ((4, 1500, 1000), "channel", "fp16dev", "aa_rows_kernel"),
+])
+def test_boxes_of_end_rows_or_short_rows_keep_one_cell_per_thread(gpu, shape, faces, storage, kernel):
+    d = Domain(*shape, storage=storage, faces=CHANNEL if faces == "channel" else ("periodic",) * 6, omega_p=1.3)
+    d.init_equilibrium()
+    try:
+        assert _step_kernels(d) == {kernel}
+    finally:
+        d.close()
+
+
 @pytest.mark.parametrize("shape,block", [((161, 2, 40), (64, 2)), ((161, 5, 40), (64, 2)), ((161, 6, 40), (64, 2)),
                                          ((161, 12, 40), (32, 4)), ((1000, 1, 3), None), ((384, 3, 9), (128, 1)), ((300, 200, 3), (32, 4))])
 def test_blocks_have_no_more_rows_than_boxes_fill(gpu, shape, block):
