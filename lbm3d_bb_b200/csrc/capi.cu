@@ -305,6 +305,20 @@ int sync_flags(lbm_ctx* c) {
   return LBM_OK;
 }
 
+// A moving body whose box holds a twenty-fifth of the nodes or more: so many warps have one of its
+// links that the kernels which send those to the general path cell by cell, or keep FP16
+// deviations across the call per link, lose (B200, us per step with poses, sphere of radius 0.12 /
+// 0.22 / 0.35 of the side: FP32 periodic 252^3 rows 524 / 782 / 1412, one cell 544 / 754 / 1272;
+// FP16 TRT channel 114^3 links on the fast path 75 / 112 / 227, general path 73 / 109 / 199).
+bool large_body(const lbm_ctx* c) {
+  if (!c->has_moving) return false;
+  const Box b = body_box(c, c->moving_body, c->pose_latest.center, 0);
+  const int n3[3] = {c->g.nx, c->g.ny, c->g.nz};
+  double nodes = 1;
+  for (int a = 0; a < 3; a++) nodes *= std::min(b.hi[a] - b.lo[a] + 1, n3[a]);
+  return 25 * nodes >= (double)c->g.N;
+}
+
 // Kinematics of a pose (lattice units as given by the caller).
 Kinematics kin_of(const lbm_pose& p) {
   Kinematics k{};
@@ -1118,9 +1132,10 @@ int32_t lbm_step(lbm_ctx* c, int32_t nsteps) {
       // up to 6 M cells, 2 M for BGK in FP16 deviations (B200, us per step, other rule / this:
       // FP32 TRT 192x96x96 87 / 72, BGK 280x150x150 218 / 216, 331x160x160 289 / 298; FP16
       // TRT 192x96x96 75 / 63, 331x160x160 273 / 281, BGK 256x128x128 130 / 146)
-      const bool bgk16 = c->cfg.storage == LBM_STORE_FP16DEV && !trt;
-      p.move = c->has_moving && has_faces(c) && !c->rows_forced && c->g.N < (bgk16 ? 2000000 : 6000000);
-      p.pair = c->pair ? 1 : (c->rows_now() && !p.move ? 2 : 0);
+      const bool bgk16 = c->cfg.storage == LBM_STORE_FP16DEV && !trt, large = large_body(c);
+      p.move = c->has_moving && has_faces(c) && !c->rows_forced && !(large && c->cfg.storage == LBM_STORE_FP16DEV) &&
+               c->g.N < (bgk16 ? 2000000 : 6000000);
+      p.pair = c->pair ? 1 : (c->rows_now() && !p.move && (c->rows_forced || !large) ? 2 : 0);
       p.quad = c->pair && c->quad ? (c->swapped ? (c->quad_odd ? 1 : 0) : (c->octo ? 2 : 1)) : 0;
       p.xshuffle = c->pair && c->xshuffle ? 1 : 0;
       if (c->tma) {

@@ -168,6 +168,30 @@ def test_boxes_of_end_rows_or_short_rows_keep_one_cell_per_thread(gpu, shape, fa
         d.close()
 
 
+@pytest.mark.parametrize("radius,faces,storage,kernel,move", [
+    (8.0, "periodic", "fp32", "aa_rows_kernel", None), (38.0, "periodic", "fp32", "aa_step_kernel", False),
+    (8.0, "channel", "fp32", "aa_step_kernel", True), (38.0, "channel", "fp32", "aa_step_kernel", True),
+    (8.0, "channel", "fp16dev", "aa_step_kernel", True), (38.0, "channel", "fp16dev", "aa_step_kernel", False)])
+def test_kernels_of_large_moving_bodies(gpu, radius, faces, storage, kernel, move):
+    """A body that fills the box keeps the general path for its links, but where the fast one wins."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    d = Domain(114, 114, 114, storage=storage, faces=CHANNEL if faces == "channel" else ("periodic",) * 6, omega_p=1.3)
+    d.add_sphere((57.0, 57.0, 57.0), radius, moving=True)
+    d.init_equilibrium()
+    try:
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            d.step(2)
+            torch.cuda.synchronize()
+        names = [e.name for e in p.events() if re.search(r"\baa_\w+_kernel\b", e.name)]
+        assert len(names) == 2 and all(kernel in name for name in names), names
+        if move is not None:  # the last template argument
+            assert all(re.search(r"(true|false)>\(", name).group(1) == str(move).lower() for name in names), names
+    finally:
+        d.close()
+
+
 @pytest.mark.parametrize("shape,block", [((161, 2, 40), (64, 2)), ((161, 5, 40), (64, 2)), ((161, 6, 40), (64, 2)),
                                          ((161, 12, 40), (32, 4)), ((1000, 1, 3), None), ((384, 3, 9), (128, 1)), ((300, 200, 3), (32, 4))])
 def test_blocks_have_no_more_rows_than_boxes_fill(gpu, shape, block):
