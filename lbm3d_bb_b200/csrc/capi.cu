@@ -283,6 +283,14 @@ int sync_flags(lbm_ctx* c) {
   r = box_union(r, body_box(c, b, c->pose_latest.center, 2));
   Box rn = dilate(r, 1);
   const bool flags_box = box_clamp(c, r), near_box = box_clamp(c, rn);
+  // One launch for small boxes, where latency counts; it evaluates the poses three times per node
+  // (a tile's surroundings too), so larger boxes take the kernels one after the other.  B200, us
+  // per step with poses, one launch / two: sphere of radius 16 in 64^3 (64 k nodes) 38.3 / 43.6,
+  // radius 20 (110 k) 69.7 / 71.6, ellipsoid of half-axis 20 60.8 / 59.4, 28 (270 k) 103.1 / 93.4,
+  // airfoil of chord 100 in 480x240x4 (250 k) 41.3 / 36.3, of 300 in 900x500x12 411 / 341.
+  bool near_due = near_box;
+  long long nodes = 1;
+  for (int a = 0; a < 3; a++) nodes *= rn.hi[a] - rn.lo[a] + 1;
   if (flags_box) {  // then rn, which holds r, is not empty
     FlagParams p{};
     p.g = c->g;
@@ -292,9 +300,13 @@ int sync_flags(lbm_ctx* c) {
     p.body_prev = to_dev(c, b, &c->pose_last_step);
     p.has_moving = 1;
     c->launches++;
-    int rc = c->cuda(geo_launch_body(p, rn, c->flags, c->links, c->stream), "moving-body flags");
+    const bool fused = nodes <= 80000;
+    int rc = c->cuda(fused ? geo_launch_body(p, rn, c->flags, c->links, c->stream) : geo_launch_moving(p, c->flags, c->stream),
+                     "moving-body flags");
     if (rc) return rc;
-  } else if (near_box) {
+    near_due = !fused;
+  }
+  if (near_due) {
     c->launches++;
     int rc = c->cuda(geo_launch_near(c->g, c->cfg.mode, rn, c->flags, c->links, c->stream), "near flags");
     if (rc) return rc;

@@ -45,3 +45,31 @@ def test_reference_mode_flags_across_the_z_ends(gpu, oracle_lib, nz, z0, kind, q
     finally:
         for d in runs:
             d.close()
+
+
+@pytest.mark.parametrize("mode,q", [("config", 19), ("reference", 19), ("reference", 27)])
+@pytest.mark.parametrize("radius,launches", [(13.0, 1), (24.0, 2)])
+def test_boxes_of_one_and_of_two_launches(gpu, oracle_lib, mode, q, radius, launches):
+    """A large body's flags come from two kernels, a small one's from one: the same rules."""
+    kw = dict(mode="reference", u_inf=(0.02, 0.0, 0.0), q=q) if mode == "reference" else dict(faces=("inlet", "outflow", "wall", "wall", "periodic", "periodic"))
+    runs = []
+    for cls, precision in ((Domain, dict(storage="fp32")), (OracleDomain, dict(precision="fp32"))):
+        d = cls(74, 66, 58, collision="BGK", omega_p=1.2, **kw, **precision)
+        d.add_body(abi.make_body(abi.BODY_SPHERE, (13.0, 12.0, 1.5), radius=4.0))
+        d.add_body(abi.make_body(abi.BODY_SPHERE, (33.2, 31.0, 50.3), radius=radius, moving=True))
+        d.init_equilibrium()
+        runs.append(d)
+    g, o = runs
+    try:
+        for n in range(1, 4):
+            pose = abi.make_pose(center=(33.2 - 0.4 * n, 31.0 + 0.3 * n, 50.3 + 1.1 * n))
+            before = g.launch_count
+            for d in runs:
+                d.update_body(pose, pose)
+                d.step(1)
+            assert g.launch_count - before == launches + 1, n
+            for a, b in zip((*g.flags(), *g.links()), (*o.flags(), *o.links())):
+                assert np.array_equal(a, b), n
+    finally:
+        for d in runs:
+            d.close()
