@@ -2320,13 +2320,28 @@ __global__ void aa_init_kernel(const InitParams p, typename SP::S* __restrict__ 
 // ---- host launch templates (instantiated once per storage policy) -------------------
 // Moments only, whole pairs (in rows for the swapped layout), output arrays on two-element words.
 // FP64 in the plain layout keeps one node per thread (256^3 433 us against 447 on B200).
+// In the swapped layout pairs on an end of the box or beside a solid read node by node, which
+// costs a warp that has one both ways.  So one node per thread serves boxes most of whose rows
+// lie on a y or z end (pairs / one node: FP16 deviations 1200x1200x1 1.05, FP64 1.16, 512x512x6
+// 0.99, FP32 0.79) and, where the x axis has faces, which then lie in every warp of short rows,
+// boxes whose rows fill the blocks (FP16 64x256x256 1.25, FP64 1.34, 256x80x80 1.22; rows that do
+// not leave lanes idle: FP64 130x256x256 0.92, FP16 34x300x150 0.71); long rows of FP32 and FP16
+// deviations gain in any case (512x256x256 0.79, 0.89; FP16 256x80x80 1.03).
 template <class SP>
-static bool export_pairs(const ReadParams& p, const ExportOut& o) {
-  if (sizeof(typename SP::S) == 8 && !p.swapped) return false;
+static bool export_pairs(const ReadParams& p, const ExportOut& o, const dim3& grid, const dim3& block) {
+  constexpr bool f64 = sizeof(typename SP::S) == 8;
+  if (f64 && !p.swapped) return false;
   const uintptr_t word = o.m_dtype == LBM_DTYPE_F64 ? 16 : 8;
   uintptr_t bits = 0;
   for (const void* a : {o.rho, o.u, o.v, o.w}) bits |= (uintptr_t)a;
-  return !o.f && bits % word == 0 && (p.swapped ? p.g.nx % 2 == 0 && p.g.nx >= 4 : p.g.N % 2 == 0);
+  if (o.f || bits % word != 0) return false;
+  const Grid& g = p.g;
+  if (!p.swapped) return g.N % 2 == 0;
+  if (g.nx % 2 != 0 || g.nx < 4) return false;
+  const double inner = (double)(g.ny > 2 ? g.ny - 2 : 0) * (g.nz > 2 ? g.nz - 2 : 0);
+  if (inner < (f64 ? 2.0 / 3.0 : 0.25) * g.ny * g.nz) return false;
+  const bool filled = 4ll * g.nx >= 3ll * grid.x * block.x;
+  return g.per[0] || !filled || (!f64 && g.nx >= (sizeof(typename SP::S) == 4 ? 128 : 384));
 }
 
 template <class SP>
@@ -2491,7 +2506,7 @@ static cudaError_t batch_sp(const BatchParams& bp, bool trt, bool force, bool fa
   }                                                                                                              \
   cudaError_t aa_export_##NAME(const ReadParams& p, const void* A, const uint8_t* flags, const ExportOut& out,   \
                                dim3 grid, dim3 block, cudaStream_t s) {                                          \
-    if (export_pairs<SP>(p, out)) return export_pair_launch<SP>(p, (const typename SP::S*)A, flags, out, s);     \
+    if (export_pairs<SP>(p, out, grid, block)) return export_pair_launch<SP>(p, (const typename SP::S*)A, flags, out, s);     \
     aa_export_kernel<SP><<<grid, block, 0, s>>>(p, (const typename SP::S*)A, flags, out);                        \
     return cudaGetLastError();                                                                                   \
   }                                                                                                              \

@@ -204,3 +204,33 @@ def test_blocks_have_no_more_rows_than_boxes_fill(gpu, shape, block):
         assert d.launch() == block
     finally:
         d.close()
+
+
+def _export_kernels(d):
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    m = torch.empty((4, (d.N + 7) // 8 * 8), device="cuda")
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        d.macros_into(*[m[k, :d.N] for k in range(4)])
+        torch.cuda.synchronize()
+    return {k for k in ("aa_export_kernel", "aa_export_pair_kernel") for e in p.events() if k in e.name}
+
+
+@pytest.mark.parametrize("shape,faces,storage,pairs", [
+    ((64, 128, 128), "channel", "fp16dev", False),   # a face in every warp
+    ((64, 128, 128), "periodic", "fp16dev", True),
+    ((34, 150, 100), "channel", "fp16dev", True),    # idle lanes in the other kernel
+    ((512, 64, 64), "channel", "fp32", True),
+    ((256, 80, 80), "channel", "fp64", False),
+    ((256, 80, 80), "periodic", "fp64", True),
+    ((600, 600, 1), "periodic", "fp64", False),      # every row on an end
+])
+def test_export_after_an_odd_number_of_steps(gpu, shape, faces, storage, pairs):
+    d = Domain(*shape, storage=storage, faces=CHANNEL if faces == "channel" else ("periodic",) * 6, omega_p=1.3)
+    d.init_equilibrium()
+    d.step(1)
+    try:
+        assert _export_kernels(d) == {"aa_export_pair_kernel" if pairs else "aa_export_kernel"}
+    finally:
+        d.close()
