@@ -2238,7 +2238,7 @@ __global__ void __launch_bounds__(256) aa_export_pair_kernel(const ReadParams p,
 }
 
 template <class SP>
-__global__ void aa_export_kernel(const ReadParams p, const typename SP::S* __restrict__ A,
+__global__ void __launch_bounds__(1024) aa_export_kernel(const ReadParams p, const typename SP::S* __restrict__ A,
                                  const uint8_t* __restrict__ flags, ExportOut out) {
   using C = typename SP::C;
   const Grid& g = p.g;
