@@ -2126,16 +2126,11 @@ __global__ void __launch_bounds__(128) aa_tma_kernel(const __grid_constant__ AAP
 // has no solid neighbour), where a look at the 18 neighbours' flags made the export 2.5 times
 // as long (512^3 FP32 5122 us against 2079 in the plain layout on B200).
 template <class SP>
-__device__ __forceinline__ void aa_read(const ReadParams& p, const typename SP::S* A, const uint8_t fl, int x, int y,
-                                        int z, long long i, typename SP::C* f) {
+__device__ __forceinline__ void aa_read_swapped(const ReadParams& p, const typename SP::S* A, const uint8_t fl, int x,
+                                                int y, int z, long long i, typename SP::C* f) {
   using C = typename SP::C;
   const Grid& g = p.g;
   const C rho0 = C(p.rho0);
-  if (!p.swapped) {
-#pragma unroll
-    for (int d = 0; d < Q; d++) f[d] = SP::ld(A + (long long)d * g.plane + i, d, rho0);
-    return;
-  }
   const uint32_t solid = (fl & F_NEAR) ? (uint32_t)((p.links[i] >> 18) & 0x3FFFFu) : 0u;
   const long long nxl = g.nx, nxy = (long long)g.nx * g.ny;
   const int xs[3] = {x == 0 ? (g.per[0] ? g.nx - 1 : -1) : x - 1, x,
@@ -2153,6 +2148,22 @@ __device__ __forceinline__ void aa_read(const ReadParams& p, const typename SP::
     }
     f[d] = SP::ld(A + a, d, rho0);
   }
+}
+
+template <class SP>
+__device__ __forceinline__ void aa_read_plain(const ReadParams& p, const typename SP::S* A, long long i,
+                                              typename SP::C* f) {
+#pragma unroll
+  for (int d = 0; d < Q; d++) f[d] = SP::ld(A + (long long)d * p.g.plane + i, d, typename SP::C(p.rho0));
+}
+
+template <class SP>
+__device__ __forceinline__ void aa_read(const ReadParams& p, const typename SP::S* A, const uint8_t fl, int x, int y,
+                                        int z, long long i, typename SP::C* f) {
+  if (p.swapped)
+    aa_read_swapped<SP>(p, A, fl, x, y, z, i, f);
+  else
+    aa_read_plain<SP>(p, A, i, f);
 }
 
 // Moments of two consecutive nodes per thread, every population without an x component (all of
@@ -2237,8 +2248,10 @@ __global__ void __launch_bounds__(256) aa_export_pair_kernel(const ReadParams p,
     }
 }
 
-template <class SP>
-__global__ void __launch_bounds__(1024) aa_export_kernel(const ReadParams p, const typename SP::S* __restrict__ A,
+// One kernel per layout: the registers of the swapped layout's addresses cost the plain one a block
+// per SM (FP64 162x100x100 60.8 us with both in one kernel, 54.6 apart).
+template <class SP, bool SWAPPED>
+__global__ void aa_export_kernel(const ReadParams p, const typename SP::S* __restrict__ A,
                                  const uint8_t* __restrict__ flags, ExportOut out) {
   using C = typename SP::C;
   const Grid& g = p.g;
@@ -2253,8 +2266,10 @@ __global__ void __launch_bounds__(1024) aa_export_kernel(const ReadParams p, con
   if (solid) {
 #pragma unroll
     for (int d = 0; d < Q; d++) f[d] = C(0);
+  } else if (SWAPPED) {
+    aa_read_swapped<SP>(p, A, fl, x, y, z, i, f);
   } else {
-    aa_read<SP>(p, A, fl, x, y, z, i, f);
+    aa_read_plain<SP>(p, A, i, f);
   }
   export_node<C>(out, g, i, f, solid, p.gacc);
 }
@@ -2507,7 +2522,8 @@ static cudaError_t batch_sp(const BatchParams& bp, bool trt, bool force, bool fa
   cudaError_t aa_export_##NAME(const ReadParams& p, const void* A, const uint8_t* flags, const ExportOut& out,   \
                                dim3 grid, dim3 block, cudaStream_t s) {                                          \
     if (export_pairs<SP>(p, out, grid, block)) return export_pair_launch<SP>(p, (const typename SP::S*)A, flags, out, s);     \
-    aa_export_kernel<SP><<<grid, block, 0, s>>>(p, (const typename SP::S*)A, flags, out);                        \
+    auto kern = p.swapped ? aa_export_kernel<SP, true> : aa_export_kernel<SP, false>;                            \
+    kern<<<grid, block, 0, s>>>(p, (const typename SP::S*)A, flags, out);                                        \
     return cudaGetLastError();                                                                                   \
   }                                                                                                              \
   cudaError_t aa_reduce_##NAME(const ReadParams& p, const void* A, const uint8_t* flags, double* out, dim3 grid, \
