@@ -40,18 +40,6 @@
 #define LBM_MINB_F16 4
 #endif
 
-// Blocks of BATCH_ITEM threads per SM that the batched kernel's register budget allows:
-// five in FP32 and FP16-deviation (96 registers), three in FP64 (168).  The kernel waits
-// for its loads, which a thread issues together only while it has registers to hold them,
-// so fewer warps with more loads in flight each win until too few warps are left.
-// Measured on B200, us per step of 8 / 16 / 64 body-fitted domains (BGK, x force):
-//   FP32   4: 38.9/93.9/430   5: 38.6/87.8/394   6: 42.5/92.7/401   7: 44.9/94.8/412
-//   FP16   5: 47.1/91.2/407   6: 48.5/98.7/407   8: 52.7/104/425
-//   FP64   3: 58.9/136/629    4: 66.2/143/645    5: 77.4/161/720
-#ifndef LBM_BATCH_MINB
-#define LBM_BATCH_MINB(SP) (sizeof(typename SP::S) == 8 ? 3 : 5)
-#endif
-
 namespace lbm {
 
 // ---- storage policies ------------------------------------------------------------
@@ -1863,8 +1851,8 @@ __device__ __forceinline__ void divmod_rcp(const unsigned n, const int d, const 
 // One kernel per phase: the ODD instance updates the domains whose phase this step is
 // odd and skips the others (both are launched every step), so each holds one phase's
 // code.
-template <class SP, bool ODD, bool TRT, int FORCE, bool FACES>
-__global__ void __launch_bounds__(BATCH_ITEM, LBM_BATCH_MINB(SP)) aa_batch_kernel(const __grid_constant__ BatchParams bp) {
+template <class SP, bool ODD, bool TRT, int FORCE, bool FACES, int BLOCKS>
+__global__ void __launch_bounds__(BATCH_ITEM, BLOCKS) aa_batch_kernel(const __grid_constant__ BatchParams bp) {
   __shared__ AAParams sp;
   using S = typename SP::S;
   const int t = threadIdx.x;
@@ -2472,12 +2460,32 @@ static cudaError_t launch_sp(const AAParams& p, void* A, const uint8_t* flags, b
   return cudaErrorInvalidValue;
 }
 
+// Blocks of BATCH_ITEM threads per SM that the batched kernel's register budget allows: five in
+// FP32 and FP16-deviation (96 registers), three in FP64 (168).  The kernel waits for its loads,
+// which a thread issues together only while it has registers to hold them, so fewer warps with
+// more loads in flight each win until too few warps are left.
+// Measured on B200, us per step of 8 / 16 / 64 body-fitted domains (BGK, x force):
+//   FP32   4: 38.9/93.9/430   5: 38.6/87.8/394   6: 42.5/92.7/401   7: 44.9/94.8/412
+//   FP16   5: 47.1/91.2/407   6: 48.5/98.7/407   8: 52.7/104/425
+//   FP64   3: 58.9/136/629    4: 66.2/143/645    5: 77.4/161/720
+// Without faces a cell waits less often, and with many items to go round more warps win:
+// 512 boxes of 16^3 (16,384 items), five / eight blocks FP16 BGK 154 / 141, TRT 165 / 151, five /
+// six FP32 TRT 159 / 152, three / four FP64 TRT 228 / 210; 32 of 32x16x16 (2048 items), five /
+// eight FP16 BGK 27 / 31.
+template <class SP, bool TRT, bool FACES>
+constexpr int batch_blocks(bool many) {
+  if (sizeof(typename SP::S) == 8) return many && !FACES && TRT ? 4 : 3;
+  if (sizeof(typename SP::S) == 4) return many && !FACES && TRT ? 6 : 5;
+  return many && !FACES ? 8 : 5;
+}
+constexpr long long BATCH_MANY = 10000;  // work items
+
 // Batched step: launches `blocks` persistent blocks, or, with per_sm != nullptr,
 // reports how many blocks of the kernel fit on one SM.
-template <class SP, bool TRT, int FORCE, bool FACES>
-static cudaError_t batch_one(const BatchParams& bp, int blocks, int* per_sm, cudaStream_t s) {
-  auto even = aa_batch_kernel<SP, false, TRT, FORCE, FACES>;
-  auto odd = aa_batch_kernel<SP, true, TRT, FORCE, FACES>;
+template <class SP, bool TRT, int FORCE, bool FACES, int BLOCKS>
+static cudaError_t batch_launch(const BatchParams& bp, int blocks, int* per_sm, cudaStream_t s) {
+  auto even = aa_batch_kernel<SP, false, TRT, FORCE, FACES, BLOCKS>;
+  auto odd = aa_batch_kernel<SP, true, TRT, FORCE, FACES, BLOCKS>;
   if (per_sm) {
     int a = 0, b = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, even, BATCH_ITEM, 0);
@@ -2490,6 +2498,14 @@ static cudaError_t batch_one(const BatchParams& bp, int blocks, int* per_sm, cud
   if (e != cudaSuccess) return e;
   odd<<<(unsigned)blocks, BATCH_ITEM, 0, s>>>(bp);
   return cudaGetLastError();
+}
+
+template <class SP, bool TRT, int FORCE, bool FACES>
+static cudaError_t batch_one(const BatchParams& bp, int blocks, int* per_sm, cudaStream_t s) {
+  constexpr int few = batch_blocks<SP, TRT, FACES>(false), many = batch_blocks<SP, TRT, FACES>(true);
+  if constexpr (many != few)
+    if (bp.items >= BATCH_MANY) return batch_launch<SP, TRT, FORCE, FACES, many>(bp, blocks, per_sm, s);
+  return batch_launch<SP, TRT, FORCE, FACES, few>(bp, blocks, per_sm, s);
 }
 
 template <class SP>

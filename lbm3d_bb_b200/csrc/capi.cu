@@ -1569,7 +1569,7 @@ int32_t lbm_batch_create(lbm_ctx* const* ctxs, int32_t count, lbm_batch** out) {
     batch_entry(b, m, b->host[m]);
   }
   int per_sm = 0, sms = 0;
-  if (b->cuda(aa_batch_blocks_per_sm(b->storage, b->trt, b->force, b->faces, &per_sm), "occupancy")) return bail(LBM_ERR_CUDA);
+  if (b->cuda(aa_batch_blocks_per_sm(b->storage, b->trt, b->force, b->faces, items, &per_sm), "occupancy")) return bail(LBM_ERR_CUDA);
   if (b->cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device), "SM count")) return bail(LBM_ERR_CUDA);
   if (per_sm < 1) return bail(b->fail(LBM_ERR_CUDA, "the batched kernel does not fit on an SM"));
   b->blocks = (int)std::min<long long>((long long)sms * per_sm, items);

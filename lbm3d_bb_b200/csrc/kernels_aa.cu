@@ -42,8 +42,9 @@ cudaError_t aa_launch_batch(int storage, const BatchParams& bp, bool trt, bool f
   return cudaErrorInvalidValue;
 }
 
-cudaError_t aa_batch_blocks_per_sm(int storage, bool trt, bool force, bool faces, int* per_sm) {
+cudaError_t aa_batch_blocks_per_sm(int storage, bool trt, bool force, bool faces, long long items, int* per_sm) {
   BatchParams none{};
+  none.items = items;
   switch (storage) {
     case LBM_STORE_FP32: return aa_batch_fp32(none, trt, force, faces, 0, per_sm, nullptr);
     case LBM_STORE_FP64: return aa_batch_fp64(none, trt, force, faces, 0, per_sm, nullptr);
