@@ -7,9 +7,10 @@ namespace lbm {
 
 // Chained launches.  A kernel begins with chain_begin(): the next kernel of the stream, launched
 // with launch_chained, may then be placed on the SMs as soon as every block here has started, and
-// waits in its own chain_begin() until this one has completed and its writes are visible.  That hides the launch latency and the ramp between dependent kernels
-// (B200, us per step: channel 96x48x48 11.4 -> 9.4, 192x96x96 TRT 60.4 -> 58.4, reference
-// 480x240x4 26.8 -> 25.2).  Launched any other way, chain_begin() does nothing.
+// waits in its own chain_begin() until this one has completed and its writes are visible.  That
+// hides the launch latency and the ramp between dependent kernels (B200, us per step: channel
+// 96x48x48 11.4 -> 9.4, 192x96x96 TRT 60.4 -> 58.4, reference 480x240x4 26.8 -> 25.2).  Launched
+// any other way, chain_begin() does nothing.
 // A kernel that allocates tensor memory triggers after its allocation: a block of the next kernel
 // that took the columns first would wait for this kernel, and this one for the columns.
 // What the kernels before it wrote, a chained kernel reads with ordinary loads: it lives from

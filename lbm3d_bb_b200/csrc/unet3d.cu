@@ -18,13 +18,13 @@
 #include <cuda.h>  // CUtensorMap and its enums (the encoder is fetched at run time)
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
-#include <mutex>
 #include <cudaTypedefs.h>
 #include <stdint.h>
 
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
+#include <mutex>
 #include <string>
 #include <type_traits>
 
@@ -237,7 +237,9 @@ __global__ void __launch_bounds__(32) tc_wait_probe_kernel(const int polls, int*
 //     9 MMAs per input plane and slice instead of 27 per output plane.
 // What bounds it: an MMA with M = 128 reads 4 KB of A and 32 N bytes of B from shared memory,
 // 33 + N / 4 cycles, against N / 2 of arithmetic; with Cout = 16 an MMA of N = 16 costs 40
-// cycles and one of N = 48, three times the work, 45.
+// cycles and one of N = 48, three times the work, 45.  The MMAs of 16 -> 16 are half of its time
+// (tensor pipe 27 %, shared memory 54 % busy): the same eight warps load a slab and then drain an
+// accumulator between two block-wide barriers.
 // Loads (cp.async, zero fill outside the box), MMAs and the epilogue of successive tiles run
 // side by side: two slabs, two accumulators, one barrier per slice.  One block per SM.
 // Measured (B200, 4 x 64 x 64 x 128 voxels): 16 -> 16 channels 592 us with the warp tiles, 52
@@ -1034,8 +1036,9 @@ __global__ void bias_grad_kernel(const bf16* dout, float* __restrict__ db, long 
 // The elementwise kernels below come in two forms.  With channels in groups of 8 and 16-byte
 // aligned tensors a thread moves whole groups (one 16-byte access each) and a block stays in one
 // row of the box, so its coordinates cost a few divisions per block instead of four 64-bit ones
-// per element; the one-element forms take everything else.  Values and their order of summation
-// are the same in both.  Measured on B200 at 4 x 64 x 64 x 128 voxels: upsampling with
+// per element; the one-element forms take everything else.  Values are the same in both, but for
+// the bias gradient and the loss, whose sums are made in another order (FP32 and FP64 rounding).
+// Measured on B200 at 4 x 64 x 64 x 128 voxels: upsampling with
 // concatenation (48 channels) 654 -> 80 us, pooling 45 -> 14 and its gradient 209 -> 32, the
 // gradient of the concatenation 197 -> 67, ReLU gradient 89 -> 25, bias gradient 63 -> 15,
 // masked loss 192 -> 30.
@@ -1969,14 +1972,13 @@ int32_t nn_pool2(const void* in, void* out, int32_t n, int32_t d, int32_t h, int
   if (!in || !out || !geo_ok(n, d, h, wd) || c <= 0 || d % 2 || h % 2 || wd % 2) return fail("nn_pool2: bad shape");
   const long long rows = (long long)n * (d / 2) * (h / 2);
   if (grouped(c, rows, in, out)) {
-    launch_chained_smem(pool2x8_kernel, row_grid(rows, wd / 2 * (c / 8)), 256, 0, (cudaStream_t)stream,
-                        (const bf16*)in, (bf16*)out,
-                                                                                       Geo{n, d, h, wd}, c);
+    launch_chained_smem(pool2x8_kernel, row_grid(rows, wd / 2 * (c / 8)), 256, 0, (cudaStream_t)stream, (const bf16*)in,
+                        (bf16*)out, Geo{n, d, h, wd}, c);
     return launched("nn_pool2");
   }
   const long long count = (long long)n * (d / 2) * (h / 2) * (wd / 2) * c;
   launch_chained_smem(pool2_kernel, blocks_for(count, 256), 256, 0, (cudaStream_t)stream, (const bf16*)in, (bf16*)out,
-                                                                          Geo{n, d, h, wd}, c, count);
+                      Geo{n, d, h, wd}, c, count);
   return launched("nn_pool2");
 }
 
@@ -1986,14 +1988,12 @@ int32_t nn_pool2_bwd(const void* dout, void* din, int32_t n, int32_t d, int32_t 
   const long long rows = (long long)n * d * h;
   if (grouped(c, rows, dout, din)) {
     launch_chained_smem(pool2x8_bwd_kernel, row_grid(rows, wd * (c / 8)), 256, 0, (cudaStream_t)stream,
-                        (const bf16*)dout, (bf16*)din,
-                                                                                       Geo{n, d, h, wd}, c, accumulate);
+                        (const bf16*)dout, (bf16*)din, Geo{n, d, h, wd}, c, accumulate);
     return launched("nn_pool2_bwd");
   }
   const long long count = (long long)n * d * h * wd * c;
   launch_chained_smem(pool2_bwd_kernel, blocks_for(count, 256), 256, 0, (cudaStream_t)stream, (const bf16*)dout,
-                      (bf16*)din,
-                                                                              Geo{n, d, h, wd}, c, accumulate, count);
+                      (bf16*)din, Geo{n, d, h, wd}, c, accumulate, count);
   return launched("nn_pool2_bwd");
 }
 
@@ -2022,14 +2022,12 @@ int32_t nn_up2_concat_bwd(const void* dcat, void* dlow, void* dskip, int32_t n, 
   if (cu % 8 == 0 && grouped(cs, rows, dcat, dlow, dskip)) {
     const int per_row = wd / 2 * (cu / 8) > wd * (cs / 8) ? wd / 2 * (cu / 8) : wd * (cs / 8);
     launch_chained_smem(up2_concat8_bwd_kernel, row_grid(rows, per_row), 256, 0, s, (const bf16*)dcat, (bf16*)dlow,
-                        (uint4*)dskip,
-                                                                   Geo{n, d, h, wd}, cu / 8, cs / 8, (unsigned)coarse);
+                        (uint4*)dskip, Geo{n, d, h, wd}, cu / 8, cs / 8, (unsigned)coarse);
     return launched("nn_up2_concat_bwd");
   }
   const long long cl = (long long)n * (d / 2) * (h / 2) * (wd / 2) * cu;
   launch_chained_smem(up2_concat_bwd_low_kernel, blocks_for(cl, 256), 256, 0, s, (const bf16*)dcat, (bf16*)dlow,
-                      Geo{n, d, h, wd}, cu,
-                                                                 cs, cl);
+                      Geo{n, d, h, wd}, cu, cs, cl);
   const long long cf = (long long)n * d * h * wd * cs;
   launch_chained_smem(up2_concat_bwd_skip_kernel, blocks_for(cf, 256), 256, 0, s, (const bf16*)dcat, (bf16*)dskip, cu,
                       cs, cf);
@@ -2044,8 +2042,7 @@ int32_t nn_mse(const void* out, const float* target, const uint8_t* mask, const 
   const auto kernel = cpad == 16 && ct == 4 && aligned16(out) && aligned16(target) && aligned16(dout) ? mse_kernel<true>
                                                                                                      : mse_kernel<false>;
   launch_chained_smem(kernel, grid, 256, 0, (cudaStream_t)stream, (const bf16*)out, target, mask, cw, (bf16*)dout,
-                      loss, voxels, cpad, ct,
-                                                 count);
+                      loss, voxels, cpad, ct, count);
   return launched("nn_mse");
 }
 
@@ -2055,8 +2052,7 @@ int32_t nn_adam(float* w, const float* g, float* m, float* v, void* wb, int64_t 
   if (count == 0) return 0;
   const float c1 = 1.f - powf(beta1, (float)t), c2 = 1.f - powf(beta2, (float)t);
   launch_chained_smem(adam_kernel, blocks_for(count, 256), 256, 0, (cudaStream_t)stream, w, g, m, v, (bf16*)wb, count,
-                      lr, beta1, beta2,
-                                                                         eps, c1, c2);
+                      lr, beta1, beta2, eps, c1, c2);
   return launched("nn_adam");
 }
 
