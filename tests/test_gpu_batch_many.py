@@ -10,6 +10,7 @@ from lbm3d_bb_b200 import Domain
 from lbm3d_bb_b200.batch import Batch
 from tests import cases
 from tests.cases import rel_l2
+from tests.kernel_names import launched
 
 pytestmark = pytest.mark.gpu
 
@@ -28,19 +29,12 @@ def _domain(k, storage, coll, faces):
 @pytest.mark.parametrize("storage,coll,few,many", [("fp16dev", "BGK", 5, 8), ("fp16dev", "TRT", 5, 8), ("fp32", "BGK", 5, 5),
                                                    ("fp32", "TRT", 5, 6), ("fp64", "BGK", 3, 3), ("fp64", "TRT", 3, 4)])
 def test_register_budget_follows_the_work(gpu, storage, coll, few, many, faces):
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-
     for count, blocks in ((4, few), (313, many if faces == cases.PERIODIC else few)):  # 32 items each
         domains = [_domain(k, storage, coll, faces) for k in range(count)]
         try:
             with Batch(domains) as b:
-                with profile(activities=[ProfilerActivity.CUDA]) as p:
-                    b.step(3)
-                    b.synchronize()
-                    torch.cuda.synchronize()
-            names = [e.name for e in p.events() if "aa_batch_kernel" in e.name]
-            assert names and {int(re.search(r", (\d+)>\(", n).group(1)) for n in names} == {blocks}, names
+                b.step(3)
+                b.synchronize()
             for k in (0, count - 1):
                 one = _domain(k, storage, coll, faces)
                 one.step(3)
@@ -49,6 +43,9 @@ def test_register_budget_follows_the_work(gpu, storage, coll, few, many, faces):
                 one.close()
                 assert rel_l2(a, c) <= TOL[storage]
                 assert np.linalg.norm(fa[:, :3] - fc[:, :3]) <= 10 * TOL[storage] * np.linalg.norm(fc[:, :3]) + 1e-12
+            with Batch(domains) as b:
+                names = launched(lambda: b.step(2), "aa_batch_kernel")
+            assert {int(re.search(r", (\d+)>\(", n).group(1)) for n in names} == {blocks}, names
         finally:
             for d in domains:
                 d.close()

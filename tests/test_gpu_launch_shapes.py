@@ -9,6 +9,7 @@ import pytest
 from lbm3d_bb_b200 import Domain
 from lbm3d_bb_b200._capi import LbmError
 from tests import cases
+from tests.kernel_names import launched
 
 pytestmark = pytest.mark.gpu
 
@@ -72,14 +73,7 @@ def test_more_rows_than_a_grid_has_blocks(gpu, storage, monkeypatch):
 
 def _step_kernels(d, steps=2):
     """Names of the step kernels that `steps` steps launch (even and odd phase)."""
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        d.step(steps)
-        torch.cuda.synchronize()
-    names = {re.sub(r".*\b(\w+_kernel)\b.*", r"\1", e.name) for e in p.events() if "_kernel" in e.name}
-    return names
+    return {re.search(r"\b(aa_\w+_kernel)\b", n).group(1) for n in launched(lambda: d.step(steps))}
 
 
 def test_a_set_shape_selects_the_one_cell_kernel(gpu):
@@ -142,7 +136,7 @@ def test_pair_variable_holds_with_a_moving_body(gpu, monkeypatch, pair, kernel):
     d = cases.moving_sphere_trt(Domain, storage="fp32")
     try:
         d.update_body(*cases.sphere_pose(d, 1))
-        assert _step_kernels(d) - {"body_flags_kernel"} == {kernel}
+        assert _step_kernels(d) == {kernel}
     finally:
         d.close()
 
@@ -174,18 +168,12 @@ def test_boxes_of_end_rows_or_short_rows_keep_one_cell_per_thread(gpu, shape, fa
     (8.0, "channel", "fp16dev", "aa_step_kernel", True), (38.0, "channel", "fp16dev", "aa_step_kernel", False)])
 def test_kernels_of_large_moving_bodies(gpu, radius, faces, storage, kernel, move):
     """A body that fills the box keeps the general path for its links, but where the fast one wins."""
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-
     d = Domain(114, 114, 114, storage=storage, faces=CHANNEL if faces == "channel" else ("periodic",) * 6, omega_p=1.3)
     d.add_sphere((57.0, 57.0, 57.0), radius, moving=True)
     d.init_equilibrium()
     try:
-        with profile(activities=[ProfilerActivity.CUDA]) as p:
-            d.step(2)
-            torch.cuda.synchronize()
-        names = [e.name for e in p.events() if re.search(r"\baa_\w+_kernel\b", e.name)]
-        assert len(names) == 2 and all(kernel in name for name in names), names
+        names = launched(lambda: d.step(2))
+        assert all(kernel in name for name in names), names
         if move is not None:  # the last template argument
             assert all(re.search(r"(true|false)>\(", name).group(1) == str(move).lower() for name in names), names
     finally:
@@ -208,13 +196,10 @@ def test_blocks_have_no_more_rows_than_boxes_fill(gpu, shape, block):
 
 def _export_kernels(d):
     import torch
-    from torch.profiler import ProfilerActivity, profile
 
     m = torch.empty((4, (d.N + 7) // 8 * 8), device="cuda")
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        d.macros_into(*[m[k, :d.N] for k in range(4)])
-        torch.cuda.synchronize()
-    return {k for k in ("aa_export_kernel", "aa_export_pair_kernel") for e in p.events() if k in e.name}
+    names = launched(lambda: d.macros_into(*[m[k, :d.N] for k in range(4)]))
+    return {k for k in ("aa_export_kernel", "aa_export_pair_kernel") for n in names if k in n}
 
 
 @pytest.mark.parametrize("shape,faces,storage,pairs", [
